@@ -169,13 +169,13 @@ def _level_state(c, seed):
         q[0] = torch.where(left, 1.0 + 0.1 * float(r[1]), 0.125)
         q[-1] = torch.where(left, 1.0 + 0.1 * float(r[2]), 0.1)
     elif D == 2:
-        # four quadrant states (rho, u, v, p), away from vacuum at walls and
-        # between receding quadrants
+        # four quadrant states (rho, u, v, p), mild enough that no limiter
+        # drives a cell into vacuum
         for k, m in enumerate([(X > 0.5) & (Y > 0.5), (X <= 0.5) & (Y > 0.5), (X <= 0.5) & (Y <= 0.5),
                                (X > 0.5) & (Y <= 0.5)]):
             m = m.expand(nz, ny, nx)
             a = [float(v) for v in r[4 * k:4 * k + 4]]
-            for n, v in enumerate((0.1 + 1.4 * a[0], 1.5 * a[1] - 0.75, 1.5 * a[2] - 0.75, 0.2 + 1.3 * a[3])):
+            for n, v in enumerate((0.5 + a[0], a[1] - 0.5, a[2] - 0.5, 0.5 + a[3])):
                 q[n][m] = v
     else:
         # a spherical blast off the middle
