@@ -85,33 +85,130 @@ __global__ void ghost_fill_kernel(int NC, const GhostOp* __restrict__ ops, int n
     }
 }
 
-// ---------------------------------------------------------------- pack
-// packed element e = cell_begin*NC + n*ncells_box + cell (always double)
-template <typename T>
-__global__ void pack_kernel(int NC, const FabDev* __restrict__ fabs, const PackBox* __restrict__ boxes, int nboxes,
-                            long long total, double* __restrict__ packed, int to_packed)
-{
-    const long long nel = total * NC;
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < nel;
-         e += (long long)gridDim.x * blockDim.x) {
-        int lo = 0, hi = nboxes - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (boxes[mid].cell_begin * NC <= e) lo = mid; else hi = mid - 1;
+// ---------------------------------------------------------------- cell walk
+// A warp's walk over consecutive cells of the packed order (box after box,
+// x fastest inside a box): lane t visits cells first + t, first + t + 32, ...
+// and knows each one's box, position in the box and fab offset.  The box is
+// searched for once per walk and then only advanced, and the position moves
+// by carrying 32 cells into the rows, so a visit costs a few integer
+// operations; one 64-bit division by the row length and two by the box per
+// element had made the pack kernel instruction bound (4096^2 FP64: 470 us
+// for 1.07 GB, 2.3 TB/s, against 164 us at the copy rate).
+struct CellWalk {
+    const PackBox* boxes;
+    const FabDev* fabs;
+    int nboxes, b, nx, ny, i, j, k;
+    long long begin, end;  // this box's cells in the packed order
+    long long off, js, ks, ns;
+
+    __device__ __forceinline__ CellWalk(const PackBox* bx, const FabDev* fb, int nb, long long c)
+        : boxes(bx), fabs(fb), nboxes(nb), b(find_by_begin(bx, nb, c))
+    {
+        enter(c);
+    }
+    __device__ __forceinline__ void enter(long long c)
+    {
+        const PackBox& B = boxes[b];
+        nx = B.hi[0] - B.lo[0] + 1;
+        ny = B.hi[1] - B.lo[1] + 1;
+        begin = B.cell_begin;
+        end = begin + (long long)nx * ny * (B.hi[2] - B.lo[2] + 1);
+        const long long local = c - begin;
+        long long row;
+        if (local >> 31) {
+            row = local / nx;
+            i = (int)(local - row * nx);
+        } else {
+            const unsigned r = (unsigned)local / (unsigned)nx;
+            i = (int)((unsigned)local - r * (unsigned)nx);
+            row = r;
         }
-        const PackBox& B = boxes[lo];
-        const int nx = B.hi[0] - B.lo[0] + 1, ny = B.hi[1] - B.lo[1] + 1, nz = B.hi[2] - B.lo[2] + 1;
-        const long long ncell = (long long)nx * ny * nz;
-        const long long local = e - B.cell_begin * NC;
-        const int n = (int)(local / ncell);
-        const long long c = local % ncell;
-        const int i = B.lo[0] + (int)(c % nx);
-        const int j = B.lo[1] + (int)((c / nx) % ny);
-        const int k = B.lo[2] + (int)(c / ((long long)nx * ny));
-        const FabDev& f = fabs[lo];
-        T* pf = f.ptr<T>() + fab_index(f, i, j, k) + n * f.ns;
-        if (to_packed) packed[e] = (double)*pf;
-        else *pf = (T)packed[e];
+        k = (int)(row / ny);
+        j = (int)(row - (long long)k * ny);
+        const FabDev& f = fabs[b];
+        js = f.js;
+        ks = f.ks;
+        ns = f.ns;
+        off = fab_index(f, B.lo[0], B.lo[1], B.lo[2]);
+    }
+    // to cell c, 32 further than the one before
+    __device__ __forceinline__ void next(long long c)
+    {
+        if (c >= end) {
+            while (b + 1 < nboxes && c >= boxes[b + 1].cell_begin) ++b;
+            enter(c);
+            return;
+        }
+        i += 32;
+        while (i >= nx) {
+            i -= nx;
+            if (++j == ny) {
+                j = 0;
+                ++k;
+            }
+        }
+    }
+    __device__ __forceinline__ long long cell() const { return off + i + j * js + k * ks; }
+    template <typename T>
+    __device__ __forceinline__ T* ptr() const { return fabs[b].ptr<T>(); }
+};
+
+constexpr int kWalkUnroll = 4;  // cells a lane holds at once
+
+// The consecutive cells [first, last) of this warp: the packed order cut
+// into equal runs of whole 32 x kWalkUnroll groups.
+__device__ __forceinline__ void walk_range(long long total, long long& first, long long& last)
+{
+    constexpr long long G = 32 * kWalkUnroll;
+    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+    const long long groups = (total + G - 1) / G;
+    const long long lo = groups * w / nw, hi = groups * (w + 1) / nw;
+    first = lo * G;
+    last = hi * G < total ? hi * G : total;
+}
+
+// ---------------------------------------------------------------- pack
+// packed element e = cell_begin*NC + n*ncells_box + cell (always double).
+// HBM bound: every value of kWalkUnroll cells is loaded before the first
+// store, 8-byte accesses of 32 consecutive cells.
+template <typename T, int NC, bool OUT>
+__global__ void __launch_bounds__(kThreads) pack_kernel(const FabDev* __restrict__ fabs, const PackBox* __restrict__ boxes, int nboxes,
+                                                        long long total, double* __restrict__ packed)
+{
+    const int lane = threadIdx.x & 31;
+    long long first, last;
+    walk_range(total, first, last);
+    if (first + lane >= last) return;
+    CellWalk w(boxes, fabs, nboxes, first + lane);
+    for (long long c0 = first + lane; c0 < last; c0 += 32 * kWalkUnroll) {
+        T v[kWalkUnroll][NC];
+        double* to_p[kWalkUnroll];
+        T* to_f[kWalkUnroll];
+        long long step[kWalkUnroll];
+#pragma unroll
+        for (int u = 0; u < kWalkUnroll; ++u) {
+            const long long c = c0 + 32 * u;
+            if (c >= last) break;
+            if (c != first + lane) w.next(c);
+            T* f = w.ptr<T>() + w.cell();
+            const long long ncell = w.end - w.begin;
+            double* p = packed + w.begin * NC + (c - w.begin);
+#pragma unroll
+            for (int n = 0; n < NC; ++n) v[u][n] = OUT ? f[n * w.ns] : (T)p[n * ncell];
+            to_p[u] = p;
+            to_f[u] = f;
+            step[u] = OUT ? ncell : w.ns;
+        }
+#pragma unroll
+        for (int u = 0; u < kWalkUnroll; ++u) {
+            if (c0 + 32 * u >= last) break;
+#pragma unroll
+            for (int n = 0; n < NC; ++n) {
+                if (OUT) to_p[u][n * step[u]] = (double)v[u][n];
+                else to_f[u][n * step[u]] = v[u][n];
+            }
+        }
     }
 }
 
@@ -150,23 +247,32 @@ __global__ void max_ws_kernel(const FabDev* __restrict__ fabs, const PackBox* __
     const K<T> k(kc);
     double wmax = 0.0;
     bool nan_seen = false;
-    for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < total;
-         c += (long long)gridDim.x * blockDim.x) {
-        const int b = find_by_begin(boxes, nboxes, c);
-        const PackBox& B = boxes[b];
-        const int nx = B.hi[0] - B.lo[0] + 1, ny = B.hi[1] - B.lo[1] + 1;
-        const long long local = c - B.cell_begin;
-        const int i = B.lo[0] + (int)(local % nx);
-        const int j = B.lo[1] + (int)((local / nx) % ny);
-        const int kk = B.lo[2] + (int)(local / ((long long)nx * ny));
-        const FabDev& f = fabs[b];
-        const T* p = f.ptr<T>() + fab_index(f, i, j, kk);
-        T U[NC];
-        for (int n = 0; n < NC; ++n) U[n] = p[n * f.ns];
-        const double w = (double)wave_speed<T, D>(U, k);
-        wmax = fmax(wmax, w);
-        nan_seen = nan_seen || (w != w);
+    const int lane = threadIdx.x & 31;
+    long long first, last;
+    walk_range(total, first, last);
+    if (first + lane < last) {
+        CellWalk w(boxes, fabs, nboxes, first + lane);
+        for (long long c0 = first + lane; c0 < last; c0 += 32 * kWalkUnroll) {
+            T U[kWalkUnroll][NC];
+#pragma unroll
+            for (int u = 0; u < kWalkUnroll; ++u) {
+                const long long c = c0 + 32 * u;
+                if (c >= last) break;
+                if (c != first + lane) w.next(c);
+                const T* p = w.ptr<T>() + w.cell();
+#pragma unroll
+                for (int n = 0; n < NC; ++n) U[u][n] = p[n * w.ns];
+            }
+#pragma unroll
+            for (int u = 0; u < kWalkUnroll; ++u) {
+                if (c0 + 32 * u >= last) break;
+                const double s = (double)wave_speed<T, D>(U[u], k);
+                wmax = fmax(wmax, s);
+                nan_seen = nan_seen || (s != s);
+            }
+        }
     }
+    __syncwarp();
     for (int off = 16; off > 0; off >>= 1) wmax = fmax(wmax, __shfl_xor_sync(0xffffffffu, wmax, off));
     const bool any_nan = __any_sync(0xffffffffu, nan_seen);
     if ((threadIdx.x & 31) == 0) {
@@ -359,14 +465,31 @@ cudaError_t launch_pack_slab(int NC, bool fp32, const FabDev& fab, const PackBox
     return cudaGetLastError();
 }
 
+template <int NC>
+static cudaError_t pack_dispatch(bool fp32, const FabDev* fabs, const PackBox* boxes, int nboxes, long long total,
+                                 double* packed, int to_packed, cudaStream_t s)
+{
+    const int g = grid_for(total, kWalkUnroll);
+    if (fp32) {
+        if (to_packed) pack_kernel<float, NC, true><<<g, kThreads, 0, s>>>(fabs, boxes, nboxes, total, packed);
+        else pack_kernel<float, NC, false><<<g, kThreads, 0, s>>>(fabs, boxes, nboxes, total, packed);
+    } else {
+        if (to_packed) pack_kernel<double, NC, true><<<g, kThreads, 0, s>>>(fabs, boxes, nboxes, total, packed);
+        else pack_kernel<double, NC, false><<<g, kThreads, 0, s>>>(fabs, boxes, nboxes, total, packed);
+    }
+    return cudaGetLastError();
+}
+
 cudaError_t launch_pack(int NC, bool fp32, const FabDev* fabs, const PackBox* boxes, int nboxes,
                         long long total_cells, double* packed, int to_packed, cudaStream_t s)
 {
     if (total_cells == 0) return cudaSuccess;
-    const int g = grid_for(total_cells * NC, 4);
-    if (fp32) pack_kernel<float><<<g, kThreads, 0, s>>>(NC, fabs, boxes, nboxes, total_cells, packed, to_packed);
-    else pack_kernel<double><<<g, kThreads, 0, s>>>(NC, fabs, boxes, nboxes, total_cells, packed, to_packed);
-    return cudaGetLastError();
+    switch (NC) {
+    case 3: return pack_dispatch<3>(fp32, fabs, boxes, nboxes, total_cells, packed, to_packed, s);
+    case 4: return pack_dispatch<4>(fp32, fabs, boxes, nboxes, total_cells, packed, to_packed, s);
+    case 5: return pack_dispatch<5>(fp32, fabs, boxes, nboxes, total_cells, packed, to_packed, s);
+    default: return cudaErrorInvalidValue;
+    }
 }
 
 template <typename T>
