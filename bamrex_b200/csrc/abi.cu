@@ -90,6 +90,8 @@ int make_consts(const bamrex_parm* p, int D, Consts& k)
         k.root_dpos_l2 = (double)(((long double)k.inv_z - (long double)kr) * 0.69314718055994530942L);
     }
     k.half_eps = 0.5 * eps;
+    k.neg_gm1_heps = -k.gm1 * k.half_eps;
+    k.one_m_gp1_2g = 1.0 - k.gp1_2g;
     k.limiter = p->limiter;
     const int NC = D + 2;
     bool uniform = true, need_prim = false;
@@ -271,12 +273,12 @@ void tma_box_items(int D, int dir, const int* lo, const int* hi, int seglen, int
 }
 
 // Steps one unit (a warp of the march, a block of the wavefront) spends on
-// a segment of len cells: the march's len + about 8 (warm-up, drain, first
-// tile); the wavefront's passes of pw positions over len + 2, plus one for
+// a segment of len cells: the march's len + 4 in whole stages of 4, plus one
+// for the first tile; the wavefront's passes of pw positions over len + 2, plus one for
 // the first tile.
 long long tma_item_cost(bool wave, int pw, int len)
 {
-    return wave ? ((long long)(len + 3 + pw - 1) / pw + 1) * pw : (long long)len + 8;
+    return wave ? ((long long)(len + 3 + pw - 1) / pw + 1) * pw : (long long)(len + 4 + 3) / 4 * 4 + 4;
 }
 
 // Segment length of a TMA-staged sweep: the candidate with the shortest
@@ -379,7 +381,7 @@ int auto_sweep_kind(int D, int d, bool fp32, const std::vector<bamrex_box>& boxe
         long long it;
         int nseg, ng, wa, bl;
         tma_box_items(D, d, b.lo, b.hi, seg_tma, 32, it, nseg, ng, wa, bl);
-        segs(seg_tma, [&](int len) { tma += (double)ng * 32 * (len + 8); });
+        segs(seg_tma, [&](int len) { tma += (double)ng * 32 * ((len + 7) / 4 * 4 + 4); });
         tma_box_items(D, d, b.lo, b.hi, seg_wave, nlw, it, nseg, ng, wa, bl);
         segs(seg_wave, [&](int len) { wave += (double)ng * nlw * ((len + 3 + pw - 1) / pw + 1) * pw; });
     }
@@ -1038,7 +1040,8 @@ extern "C" int bamrex_level_create(bamrex_level** out, const bamrex_level_desc* 
         return fail(BAMREX_ERR_ARG, "staging must be BAMREX_STAGING_AUTO, _REGISTERS, _TMA or _WAVE");
     }
     {
-        const bool ok = tma_supported(D, L->method, L->k);
+        const bool fast = tma_supported(D, L->method, L->k);
+        const bool ok = fast || (D >= 2 && tma_requestable(D, L->method, L->k));
         if ((desc->staging == BAMREX_STAGING_TMA || desc->staging == BAMREX_STAGING_WAVE) && !ok) {
             delete L;
             return fail(BAMREX_ERR_UNSUPPORTED, "TMA staging needs the fast MUSCL-Hancock path (energy limiting, "
@@ -1055,7 +1058,8 @@ extern "C" int bamrex_level_create(bamrex_level** out, const bamrex_level_desc* 
                 return fail(BAMREX_ERR_UNSUPPORTED, "TMA staging needs the fast MUSCL-Hancock path (energy limiting, "
                                                     "gamma 1.4) in 2D or 3D");
             }
-            L->sweep_kind[d] = want == BAMREX_STAGING_AUTO ? -1 : want;  // -1: decided below by the cost model
+            // -1: decided below by the cost model
+            L->sweep_kind[d] = want == BAMREX_STAGING_AUTO ? -1 : fast ? want : BAMREX_STAGING_REGISTERS;
         }
     }
 
@@ -1857,7 +1861,7 @@ extern "C" int bamrex_level_est_time_step(bamrex_level* L, double* dt_est)
     if (!L->ws_valid) {
         cudaError_t e = cudaMemsetAsync(&L->d_scal->ws_bits, 0, sizeof(unsigned long long), L->stream);
         if (e != cudaSuccess) return L->set_err(cuda_fail(e, "memset"));
-        BX_TRY(level_launch(L, launch_max_wave_speed(L->D, L->fp32, L->d_fab[L->cur], L->d_pack, (int)L->boxes.size(), L->ncells, L->k,
+        BX_TRY(level_launch(L, launch_max_wave_speed(L->D, L->fp32, fast_limiter(L->D, L->method, L->k) >= 0, L->d_fab[L->cur], L->d_pack, (int)L->boxes.size(), L->ncells, L->k,
                                                      &L->d_scal->ws_bits, nullptr, L->stream),
                             "max wave speed"));
     }
@@ -1896,7 +1900,7 @@ extern "C" int bamrex_level_run_async(bamrex_level* L, int nsteps, double stop_t
     cudaError_t e = cudaMemcpyAsync(L->d_scal, h, sizeof(StepScalars), cudaMemcpyHostToDevice, L->stream);
     if (e != cudaSuccess) return L->set_err(cuda_fail(e, "scalars upload"));
     // computeInitialDt from the current state
-    BX_TRY(level_launch(L, launch_max_wave_speed(L->D, L->fp32, L->d_fab[L->cur], L->d_pack, (int)L->boxes.size(), L->ncells, L->k,
+    BX_TRY(level_launch(L, launch_max_wave_speed(L->D, L->fp32, fast_limiter(L->D, L->method, L->k) >= 0, L->d_fab[L->cur], L->d_pack, (int)L->boxes.size(), L->ncells, L->k,
                                                  &L->d_scal->ws_bits, L->d_scal, L->stream),
                         "max wave speed"));
     BX_TRY(level_launch(L, launch_step_dt(L->d_scal, L->D, L->dx[0], L->dx[1], L->dx[2], L->cfl, 0, L->stream), "step dt"));

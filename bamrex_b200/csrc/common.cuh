@@ -32,6 +32,8 @@ struct Consts {
     double root_dneg_l2;   // root_dneg * ln 2 (applied to log2 x)
     double root_dpos_l2;   // root_dpos * ln 2
     double half_eps;       // 0.5 * epsilon
+    double neg_gm1_heps;   // -(gamma - 1) * half_eps
+    double one_m_gp1_2g;   // 1 - gp1_2g
     int limiter;        // BAMREX_MINBEE ..
     // Limiting variable per component (Parm::limiter_indices /
     // limit_on_primv, Source/Fluxes/CalcLimitingVal.H:9-22).  uniform_var >= 0

@@ -27,6 +27,7 @@ constexpr double kMinP = 1e-14;
 template <typename T>
 struct K {
     T gamma, eps, inv_eps, gm1, half_gm1, z, neg_z, inv_z, gp1_2g, gamma_inv_eps, half_eps;
+    T neg_gm1_heps, one_m_gp1_2g;  // -(gamma - 1) eps / 2 and 1 - (gamma + 1) / (2 gamma): the fast path
     double root_dneg_l2, root_dpos_l2;
     int root_k, limiter, uniform_var, need_prim;
     int lim_var[kMaxComp], lim_prim[kMaxComp];
@@ -34,7 +35,8 @@ struct K {
     __device__ __forceinline__ explicit K(const Consts& c)
         : gamma((T)c.gamma), eps((T)c.eps), inv_eps((T)c.inv_eps), gm1((T)c.gm1), half_gm1((T)c.half_gm1),
           z((T)c.z), neg_z((T)c.neg_z), inv_z((T)c.inv_z), gp1_2g((T)c.gp1_2g), gamma_inv_eps((T)c.gamma_inv_eps),
-          half_eps((T)c.half_eps), root_dneg_l2(c.root_dneg_l2), root_dpos_l2(c.root_dpos_l2), root_k(c.root_k),
+          half_eps((T)c.half_eps), neg_gm1_heps((T)c.neg_gm1_heps), one_m_gp1_2g((T)c.one_m_gp1_2g),
+          root_dneg_l2(c.root_dneg_l2), root_dpos_l2(c.root_dpos_l2), root_k(c.root_k),
           limiter(c.limiter), uniform_var(c.uniform_var), need_prim(c.need_prim)
     {
 #pragma unroll
@@ -361,7 +363,6 @@ __device__ __forceinline__ float sqrt_fast(float x)
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-__device__ __forceinline__ double sqrt_fast(double x) { return sqrt(x); }
 
 // sqrt(x) for a positive, normal, finite x without the special-case branch of
 // sqrt(): the coupled iteration for g ~ sqrt(x), h ~ 1 / (2 sqrt(x)) seeded
@@ -369,33 +370,21 @@ __device__ __forceinline__ double sqrt_fast(double x) { return sqrt(x); }
 // error below 2^-19.9): one step g += g r with r = 1/2 - g h (relative error
 // ~1.5 e^2, e the seed's), then the correction g += h (x - g^2) with the
 // seed's h, whose own error only scales the already tiny correction
-// (P. Markstein, IA-64 and Elementary Functions, 2000).  Zero, infinity and
-// subnormal x give NaN.  FP32: the hardware approximation.
+// (P. Markstein, IA-64 and Elementary Functions, 2000).  The seed is halved
+// in its exponent field (an integer subtraction, off the FP64 pipe).  Zero,
+// infinity and subnormal x give NaN.
 __device__ __forceinline__ double sqrt_pos(double x)
 {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double g = x * y, h = 0.5 * y;
+    const double g = x * y;
+    const double h = __hiloint2double(__double2hiint(y) - 0x00100000, __double2loint(y));
     const double r = fma(-g, h, 0.5);
     const double g1 = fma(g, r, g);
     const double d = fma(-g1, g1, x);
     return fma(d, h, g1);
 }
-__device__ __forceinline__ float sqrt_pos(float x) { return sqrt_fast(x); }
 
-// sqrt(x) for every x with the IEEE special results (0 for 0, +inf for
-// +inf, NaN for negative or NaN x), branch-free: subnormal x are scaled by
-// 2^108 into the normal range before sqrt_pos and the root by 2^-54 after.
-// Within one ulp of the correctly rounded root (sqrt_pos itself matched it
-// on every one of 5e7 probed normal arguments).
-__device__ __forceinline__ double sqrt_any(double x)
-{
-    const bool tiny = x < 0x1p-1022;
-    const double r = sqrt_pos(tiny ? x * 0x1p108 : x);
-    const double rs = tiny ? r * 0x1p-54 : r;
-    return (x == 0.0 || x == __longlong_as_double(0x7ff0000000000000LL)) ? x : rs;
-}
-__device__ __forceinline__ float sqrt_any(float x) { return sqrt_fast(x); }
 __device__ __forceinline__ float ex2_fast(float x)
 {
     float r;
@@ -409,76 +398,240 @@ __device__ __forceinline__ float lg2_fast(float x)
     return r;
 }
 
-// log2|x| in single precision from the exponent bits and the mantissa; valid
-// over the whole normal double range (no float overflow).
-__device__ __forceinline__ float log2_abs(double x)
+// log2(x) of a positive normal double in single precision from its exponent
+// field and the first 20 mantissa bits (absolute error below 2^-19 for the
+// mantissa part): integer operations and one lg2, no conversion.
+__device__ __forceinline__ float log2_hi(double x)
 {
-    const long long bits = __double_as_longlong(x);
-    const int ex = (int)((bits >> 52) & 0x7ff) - 1023;
-    const double m = __longlong_as_double((bits & 0x000fffffffffffffLL) | 0x3ff0000000000000LL);
-    return (float)ex + __log2f((float)m);
+    const int hi = __double2hiint(x);
+    const float ex = __int_as_float(0x4b400000 + ((hi >> 20) & 0x7ff)) - (12582912.0f + 1023.0f);
+    return ex + lg2_fast(__int_as_float(0x3f800000 | ((hi & 0x000fffff) << 3)));
 }
 
-// x^(-z) with 1/z ~ 7 for x >= 1e-14 (HLLC.H:272), and 1/x as a by-product.
-// FP64: seed y0 = 2^(-log2(x)/7) in single precision (the hardware
-// approximations of log2 and exp2, a few ulp), then one step of the series
-// of (1 - e)^(-1/7), e = 1 - x y0^7 (third-order convergence: |e| ~ 2e-6
-// leaves ~5e-19), then the factor x^(1/7 - z) ~ 1 + (1/7 - z) ln x;
-// 1/x = y0^7 / (1 - e) ~ y0^7 (1 + e + e^2).  FP32: exp2(-z log2 x) on the
-// special-function unit.
-__device__ __forceinline__ void root7_neg_z(double x, const K<double>& c, double& y, double& inv_x)
+// w^(-1/7) and 1/w for a positive normal w.  FP64: seed y0 = 2^(-log2(w)/7)
+// in single precision (relative error below 2^-20; its bits are moved into a
+// double by integer operations), then one step of the series of
+// (1 - e)^(-1/7), e = 1 - w y0^7 (third-order convergence: |e| < 2^-17 leaves
+// ~1e-17); 1/w = y0^7 / (1 - e) ~ y0^7 (1 + e + e^2).
+__device__ __forceinline__ void root7(double w, double& y, double& inv_w)
 {
-    const float lf = log2_abs(x);
-    const float q = -lf * (1.0f / 7.0f);
-    const float qi = floorf(q);
-    const double p2 = __longlong_as_double((long long)((int)qi + 1023) << 52);
-    const double y0 = p2 * (double)ex2_fast(q - qi);
+    const float q = log2_hi(w) * (-1.0f / 7.0f);
+    const float qr = q + 12582912.0f;  // the nearest integer in the low mantissa bits
+    const int n = __float_as_int(qr);
+    const int f = __float_as_int(ex2_fast(q - (qr - 12582912.0f)));  // 2^[-1/2, 1/2]
+    const double y0 = __hiloint2double((f >> 3) + ((1023 - 127) << 20) + ((n - 0x4b400000) << 20), f << 29);
     const double y2 = y0 * y0, y3 = y2 * y0, y6 = y3 * y3, y7 = y6 * y0;
-    const double e = fma(-x, y7, 1.0);
-    const double t = e * fma(e, 8.0 / 98.0, 1.0 / 7.0);
-    y = fma(y0, t + c.root_dneg_l2 * (double)lf, y0);
-    inv_x = fma(y7, fma(e, e, e), y7);
+    const double e = fma(-w, y7, 1.0);
+    y = fma(y0, e * fma(e, 8.0 / 98.0, 1.0 / 7.0), y0);
+    inv_w = fma(y7, fma(e, e, e), y7);
 }
-__device__ __forceinline__ void root7_neg_z(float x, const K<float>& c, float& y, float& inv_x)
+
+// b^7 = p_rr / p_L from the two-rarefaction estimate's base b (1/z = 7 to
+// within 1e-14 on the fast path, which moves b^(1/z) by less than an ulp or
+// two; the rounding of b alone moves b^7 by as much).  A negative base gives
+// a negative result (the reference's pow gives NaN there); both make every
+// "p_rr > p_K" test false, so the wave speeds agree.
+__device__ __forceinline__ double pow7(double b)
+{
+    const double b2 = b * b, b3 = b2 * b, b6 = b3 * b3;
+    return b6 * b;
+}
+
+// Velocities, pressure and 1/rho, and mn un (the advected normal momentum,
+// shared by the kinetic energy and the flux): p = (gamma-1) E - (gamma-1)
+// eps/2 (m . u).
+template <int D, int DIR>
+struct Prim {
+    double ir, u[D], p, mnu;
+    __device__ __forceinline__ Prim(const double (&U)[D + 2], const K<double>& k)
+    {
+        ir = rcp_fast(U[0]);
+#pragma unroll
+        for (int d = 0; d < D; ++d) u[d] = U[1 + d] * ir;
+        mnu = U[1 + DIR] * u[DIR];
+        double mu = mnu;
+#pragma unroll
+        for (int d = 0; d < D; ++d)
+            if (d != DIR) mu = fma(U[1 + d], u[d], mu);
+        p = fma(k.neg_gm1_heps, mu, k.gm1 * U[1 + D]);
+    }
+};
+
+__device__ __forceinline__ bool both_zero(double a, double b)
+{
+    return (((unsigned)(__double2hiint(a) | __double2hiint(b)) << 1) | (unsigned)(__double2loint(a) | __double2loint(b))) == 0u;
+}
+__device__ __forceinline__ bool same_sign(double a, double b) { return (__double2hiint(a) ^ __double2hiint(b)) >= 0; }
+__device__ __forceinline__ bool neg_bit(double a) { return __double2hiint(a) < 0; }
+__device__ __forceinline__ bool at_least_one(double a) { return __double2hiint(a) >= 0x3ff00000; }
+
+// A quarter of the limiter value of Flux_Helpers.cpp:103-111 and
+// Limiters.H:29-73 without branches; sum = num + den.  With r = num / den
+// every limiter is, for r > 0, a single quotient whose operands the case of
+// r selects (minbee: num / den for r <= 1, 2 den / sum above; van Leer: 2
+// min-side / sum; van Albada: num sum / (num^2 + den^2) for r <= 1, 2 den /
+// sum above; superbee: 2 num / den, 1, 2 den / sum), so it takes one
+// reciprocal; the cases are decided from num and den exactly (r > 1 is |num|
+// > |den| with equal signs; the sign tests are integer ones).
+template <int LIM>
+__device__ __forceinline__ double quarter_limiter(double num, double den, double sum)
+{
+    const double an = fabs(num), ad = fabs(den);
+    const bool big = an > ad;
+    double phi;
+    if constexpr (LIM == LIM_MINBEE) {
+        const double q = (big ? den : num) * rcp_fast(big ? sum : den);
+        phi = q * (big ? 0.5 : 0.25);
+    } else if constexpr (LIM == LIM_VAN_LEER) {
+        phi = 0.5 * (big ? den : num) * rcp_fast(sum);
+    } else if constexpr (LIM == LIM_VAN_ALBADA) {
+        const double q = (big ? den : num * sum) * rcp_fast(big ? sum : fma(num, num, den * den));
+        phi = q * (big ? 0.5 : 0.25);
+    } else {
+        const bool half = 2.0 * an <= ad;
+        const double q = 0.5 * (big ? den : num) * rcp_fast(big ? sum : den);
+        phi = (half || big) ? q : 0.25;
+    }
+    phi = same_sign(num, den) ? phi : 0.0;
+    return both_zero(num, den) ? 0.25 : phi;
+}
+
+template <int D, int DIR, int LIM>
+__device__ __forceinline__ void muscl_cell_f64(const double (&Um)[D + 2], const double (&U0)[D + 2], const double (&Up)[D + 2],
+                                                const K<double>& k, double hdtdx, double (&UL)[D + 2], double (&UR)[D + 2])
+{
+    constexpr int NC = D + 2;
+    constexpr int E = D + 1;
+    // 0.5 phi delta with delta = 0.5 (U0 - Um) + 0.5 (Up - U0) written as
+    // 0.25 phi (Up - Um) (within an ulp of the reference's rounding)
+    double d2[NC];
+#pragma unroll
+    for (int n = 0; n < NC; ++n) d2[n] = Up[n] - Um[n];
+    const double qphi = quarter_limiter<LIM>(U0[E] - Um[E], Up[E] - U0[E], d2[E]);
+#pragma unroll
+    for (int n = 0; n < NC; ++n) {
+        UL[n] = fma(-qphi, d2[n], U0[n]);
+        UR[n] = fma(qphi, d2[n], U0[n]);
+    }
+    // the half step by the difference of the two physical fluxes
+    const Prim<D, DIR> a(UL, k), b(UR, k);
+    double dF[NC];
+    dF[0] = UR[1 + DIR] - UL[1 + DIR];
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+        dF[1 + d] = d == DIR ? fma(b.p - a.p, k.inv_eps, b.mnu - a.mnu)
+                             : fma(UR[1 + DIR], b.u[d], -(UL[1 + DIR] * a.u[d]));
+    dF[E] = fma(UR[E] + b.p, b.u[DIR], -((UL[E] + a.p) * a.u[DIR]));
+#pragma unroll
+    for (int n = 0; n < NC; ++n) {
+        UL[n] = fma(-hdtdx, dF[n], UL[n]);
+        UR[n] = fma(-hdtdx, dF[n], UR[n]);
+    }
+}
+
+// HLLC (hllc_face above, HLLC.cpp:90-172 with HLLC.H:214-337), rearranged to
+// spend fewer operations on the FP64 pipe, which bounds the sweeps:
+//  * the two-rarefaction pressure as a ratio: p_rr / p_L = b^(1/z) with b =
+//    (c_L + c_R - (gamma-1)/2 (u_R - u_L)) / (c_L + c_R (p_L/p_R)^z), so one
+//    seventh root serves both sides, and p_rr / p_R = (p_rr / p_L)(p_L / p_R)
+//    comes out of the same iteration;
+//  * with a_K = c_K q_K > 0 the speeds are S_L = u_L - a_L, S_R = u_R + a_R,
+//    and S* = ((p_L - p_R)/eps + m_L u_L + m_R u_R) / (m_L + m_R), m_K =
+//    rho_K a_K;
+//  * the star flux in advective form: rho* = rho_K (S_K - u_K)/(S_K - S*),
+//    p* = p_K + eps rho_K (S_K - u_K)(S* - u_K), E* from the energy jump, F =
+//    S* (rho*, rho* u*, E* + p*) + p*/eps; with u_K in place of S* the same
+//    expressions give rho_K, p_K and E_K, so they are the supersonic flux.
+template <int D, int DIR>
+__device__ __forceinline__ void hllc_face_f64(const double (&L)[D + 2], const double (&R)[D + 2], const K<double>& k,
+                                               double (&F)[D + 2])
+{
+    constexpr int E = D + 1;
+    const Prim<D, DIR> l(L, k), r(R, k);
+    // the estimate's clamped density and pressure (HLLC.H:255-260)
+    const bool okL = L[0] >= kMinRho, okR = R[0] >= kMinRho;
+    const double rhoL = okL ? L[0] : kMinRho, rhoR = okR ? R[0] : kMinRho;
+    const double icL = okL ? l.ir : 1.0 / kMinRho, icR = okR ? r.ir : 1.0 / kMinRho;
+    const double pL = l.p >= kMinP ? l.p : kMinP, pR = r.p >= kMinP ? r.p : kMinP;
+    const double uL = l.u[DIR], uR = r.u[DIR];
+    // positive arguments: p >= 1e-14 and 1 / rho <= 1e14 (clamped above)
+    const double cL = sqrt_pos(k.gamma_inv_eps * pL * icL);
+    const double cR = sqrt_pos(k.gamma_inv_eps * pR * icR);
+    double t, p_lr;  // (p_L / p_R)^z and p_L / p_R
+    root7(pR * rcp_fast(pL), t, p_lr);
+    const double rrL = pow7(fma(-k.half_gm1, uR - uL, cL + cR) * rcp_fast(fma(cR, t, cL)));
+    const double rrR = rrL * p_lr;
+    // q_K = sqrt(1 + (gamma+1)/(2 gamma) (max(p_rr / p_K, 1) - 1)): the select
+    // is on the argument (whose value at 1 is exactly 1), since a select
+    // between a root and 1 becomes a branch around the root
+    const double aL = cL * sqrt_pos(fma(k.gp1_2g, at_least_one(rrL) ? rrL : 1.0, k.one_m_gp1_2g));
+    const double aR = cR * sqrt_pos(fma(k.gp1_2g, at_least_one(rrR) ? rrR : 1.0, k.one_m_gp1_2g));
+    const double SL = uL - aL, SR = uR + aR;
+    const double mL = rhoL * aL, mR = rhoR * aR;
+    const double Ss = fma(mL, uL, fma(mR, uR, (pL - pR) * k.inv_eps)) * rcp_fast(mL + mR);
+
+    // left states when S_L >= 0 or S* >= 0, right ones otherwise; supersonic
+    // when S_L >= 0 or S_R < 0 (sign bits)
+    const bool useL = !(neg_bit(SL) && neg_bit(Ss));
+    const bool star = useL ? neg_bit(SL) : !neg_bit(SR);
+    const double un = useL ? uL : uR, p = useL ? l.p : r.p, en = useL ? L[E] : R[E];
+    const double SK = useL ? SL : SR, dK = useL ? -aL : aR;
+    const double us = star ? Ss : un;
+    const double m = (useL ? L[0] : R[0]) * dK;
+    const double rb = rcp_fast(SK - us);
+    const double ps = fma(m * k.eps, us - un, p);
+    const double es = fma(ps, us, fma(-p, un, en * dK)) * rb;
+    const double mass = m * rb * us;
+    F[0] = mass;
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+        F[1 + d] = d == DIR ? fma(mass, us, ps * k.inv_eps) : mass * (useL ? l.u[d] : r.u[d]);
+    F[E] = us * (es + ps);
+}
+
+// |u| + c, within a few ulp; NaN for a negative pressure or density, as the
+// roots are.  Both radicands are offset by 1e-300: exact for every normal
+// value above 1e-284, and a fluid at rest (or without pressure) adds 1e-150
+// instead of 0, which the sum's rounding drops unless both vanish (reduce_ws
+// takes such a maximum back to 0).
+template <int D>
+__device__ __forceinline__ double wave_speed_f64(const double (&U)[D + 2], const K<double>& k)
+{
+    const Prim<D, 0> q(U, k);
+    double mu = q.mnu;
+#pragma unroll
+    for (int d = 1; d < D; ++d) mu = fma(U[1 + d], q.u[d], mu);
+    return sqrt_pos(fma(k.gamma_inv_eps * q.p, q.ir, 1e-300)) + sqrt_pos(fma(mu, q.ir, 1e-300));
+}
+
+// ---- FP32 storage: the same scheme with the hardware approximations -------
+
+// x^(-z) (HLLC.H:272) and 1/x on the special-function unit.
+__device__ __forceinline__ void root7_neg_z_f32(float x, const K<float>& c, float& y, float& inv_x)
 {
     y = ex2_fast(c.neg_z * lg2_fast(x));
     inv_x = rcp_fast(x);
 }
 
-// b^(1/z) with 1/z = 7 + dpos: b^7 (1 + dpos ln b).  A negative base gives a
-// negative result (the reference's pow gives NaN there); both make every
-// "p_rr > p_K" test false, so the wave speeds agree.  FP32: exp2(log2(b)/z)
-// (NaN for a negative base, as the reference).
-__device__ __forceinline__ double pow7_inv_z(double b, const K<double>& c)
-{
-    const double b2 = b * b, b3 = b2 * b, b6 = b3 * b3, b7 = b6 * b;
-    return fma(b7, c.root_dpos_l2 * (double)log2_abs(b), b7);
-}
-__device__ __forceinline__ float pow7_inv_z(float b, const K<float>& c)
-{
-    // lg2 of a negative base is NaN, as the reference's pow
-    return ex2_fast(c.inv_z * lg2_fast(b));
-}
-
-template <typename T, int D>
-__device__ __forceinline__ void to_prim_fast(const T (&U)[D + 2], const K<T>& k, T (&q)[D + 2], T& inv_rho)
+template <int D>
+__device__ __forceinline__ void to_prim_f32(const float (&U)[D + 2], const K<float>& k, float (&q)[D + 2], float& inv_rho)
 {
     inv_rho = rcp_fast(U[0]);
     q[0] = U[0];
 #pragma unroll
     for (int d = 0; d < D; ++d) q[1 + d] = U[1 + d] * inv_rho;
-    T usq = q[1] * q[1];
+    float usq = q[1] * q[1];
 #pragma unroll
     for (int d = 1; d < D; ++d) usq = usq + q[1 + d] * q[1 + d];
     q[1 + D] = k.gm1 * (U[1 + D] - k.half_eps * U[0] * usq);
 }
 
-template <typename T, int D, int DIR>
-__device__ __forceinline__ void phys_flux_fast(const T (&U)[D + 2], const K<T>& k, T (&F)[D + 2])
+template <int D, int DIR>
+__device__ __forceinline__ void phys_flux_f32(const float (&U)[D + 2], const K<float>& k, float (&F)[D + 2])
 {
-    T q[D + 2], ir;
-    to_prim_fast<T, D>(U, k, q, ir);
-    phys_flux<T, D, DIR>(U, q, k, F);
+    float q[D + 2], ir;
+    to_prim_f32<D>(U, k, q, ir);
+    phys_flux<float, D, DIR>(U, q, k, F);
 }
 
 // The limiter value of Flux_Helpers.cpp:103-111 and Limiters.H:29-73 without
@@ -490,125 +643,125 @@ __device__ __forceinline__ void phys_flux_fast(const T (&U)[D + 2], const K<T>& 
 // exactly (r > 1 is |num| > |den| with equal signs), which agrees with the
 // rounded quotient except where that rounds to exactly 1 or 1/2, and there
 // both formulas give the same value to an ulp.
-template <typename T, int LIM>
-__device__ __forceinline__ T limiter_value_fast(T num, T den)
+template <int LIM>
+__device__ __forceinline__ float limiter_value_f32(float num, float den)
 {
-    const bool pos = (num > T(0) && den > T(0)) || (num < T(0) && den < T(0));  // r > 0
-    const T an = fabs(num), ad = fabs(den);
-    T phi;
+    const bool pos = (num > 0.0f && den > 0.0f) || (num < 0.0f && den < 0.0f);  // r > 0
+    const float an = fabs(num), ad = fabs(den);
+    float phi;
     if constexpr (LIM == LIM_MINBEE) {
         const bool big = an > ad;  // r > 1
-        phi = (big ? T(2) * den : num) * rcp_fast(big ? den + num : den);
+        phi = (big ? 2.0f * den : num) * rcp_fast(big ? den + num : den);
     } else if constexpr (LIM == LIM_VAN_LEER) {
         // 2 r / (1 + r) for r <= 1, 2 / (1 + r) above
-        phi = T(2) * (an > ad ? den : num) * rcp_fast(den + num);
+        phi = 2.0f * (an > ad ? den : num) * rcp_fast(den + num);
     } else if constexpr (LIM == LIM_VAN_ALBADA) {
-        const T r = num * rcp_fast(den);
-        phi = fmin(r * (T(1) + r) * rcp_fast(T(1) + r * r), T(2) * rcp_fast(T(1) + r));
+        const float r = num * rcp_fast(den);
+        phi = fmin(r * (1.0f + r) * rcp_fast(1.0f + r * r), 2.0f * rcp_fast(1.0f + r));
     } else {
         // 2 r for r <= 1/2, 1 for r <= 1, min(r, 2 / (1 + r), 2) = 2 / (1 + r) above
-        const bool big = an > ad, half = T(2) * an <= ad;
-        const T q = (big ? T(2) * den : T(2) * num) * rcp_fast(big ? den + num : den);
-        phi = (half || big) ? q : T(1);
+        const bool big = an > ad, half = 2.0f * an <= ad;
+        const float q = (big ? 2.0f * den : 2.0f * num) * rcp_fast(big ? den + num : den);
+        phi = (half || big) ? q : 1.0f;
     }
-    phi = pos ? phi : T(0);
-    return (num == T(0) && den == T(0)) ? T(1) : phi;
+    phi = pos ? phi : 0.0f;
+    return (num == 0.0f && den == 0.0f) ? 1.0f : phi;
 }
 
-template <typename T, int D, int DIR, int LIM>
-__device__ __forceinline__ void muscl_cell_fast(const T (&Um)[D + 2], const T (&U0)[D + 2], const T (&Up)[D + 2],
-                                                const K<T>& k, T hdtdx, T (&UL)[D + 2], T (&UR)[D + 2])
+template <int D, int DIR, int LIM>
+__device__ __forceinline__ void muscl_cell_f32(const float (&Um)[D + 2], const float (&U0)[D + 2], const float (&Up)[D + 2],
+                                                const K<float>& k, float hdtdx, float (&UL)[D + 2], float (&UR)[D + 2])
 {
     constexpr int NC = D + 2;
     constexpr int E = D + 1;
     // 0.5 phi delta with delta = 0.5 (U0 - Um) + 0.5 (Up - U0) written as
     // 0.25 phi (Up - Um) (within an ulp of the reference's rounding)
-    const T qphi = T(0.25) * limiter_value_fast<T, LIM>(U0[E] - Um[E], Up[E] - U0[E]);
+    const float qphi = 0.25f * limiter_value_f32<LIM>(U0[E] - Um[E], Up[E] - U0[E]);
 #pragma unroll
     for (int n = 0; n < NC; ++n) {
-        const T d2 = Up[n] - Um[n];
+        const float d2 = Up[n] - Um[n];
         UL[n] = fma(-qphi, d2, U0[n]);
         UR[n] = fma(qphi, d2, U0[n]);
     }
-    T FL[NC], FR[NC];
-    phys_flux_fast<T, D, DIR>(UL, k, FL);
-    phys_flux_fast<T, D, DIR>(UR, k, FR);
+    float FL[NC], FR[NC];
+    phys_flux_f32<D, DIR>(UL, k, FL);
+    phys_flux_f32<D, DIR>(UR, k, FR);
 #pragma unroll
     for (int n = 0; n < NC; ++n) {
-        const T dF = hdtdx * (FR[n] - FL[n]);
+        const float dF = hdtdx * (FR[n] - FL[n]);
         UL[n] -= dF;
         UR[n] -= dF;
     }
 }
 
-template <typename T, int D, int DIR>
-__device__ __forceinline__ void hllc_face_fast(const T (&L)[D + 2], const T (&R)[D + 2], const K<T>& k,
-                                               T (&F)[D + 2])
+template <int D, int DIR>
+__device__ __forceinline__ void hllc_face_f32(const float (&L)[D + 2], const float (&R)[D + 2], const K<float>& k,
+                                               float (&F)[D + 2])
 {
     constexpr int NC = D + 2;
-    T qL[NC], qR[NC], irL, irR;
-    to_prim_fast<T, D>(L, k, qL, irL);
-    to_prim_fast<T, D>(R, k, qR, irR);
-    const T rhoL = fmax(qL[0], T(kMinRho)), rhoR = fmax(qR[0], T(kMinRho));
-    const T pL = fmax(qL[1 + D], T(kMinP)), pR = fmax(qR[1 + D], T(kMinP));
-    const T uL = qL[1 + DIR], uR = qR[1 + DIR];
-    const T icL = (qL[0] >= T(kMinRho)) ? irL : T(1.0 / kMinRho);
-    const T icR = (qR[0] >= T(kMinRho)) ? irR : T(1.0 / kMinRho);
+    float qL[NC], qR[NC], irL, irR;
+    to_prim_f32<D>(L, k, qL, irL);
+    to_prim_f32<D>(R, k, qR, irR);
+    const float rhoL = fmax(qL[0], (float)kMinRho), rhoR = fmax(qR[0], (float)kMinRho);
+    const float pL = fmax(qL[1 + D], (float)kMinP), pR = fmax(qR[1 + D], (float)kMinP);
+    const float uL = qL[1 + DIR], uR = qR[1 + DIR];
+    const float icL = (qL[0] >= (float)kMinRho) ? irL : (float)(1.0 / kMinRho);
+    const float icR = (qR[0] >= (float)kMinRho) ? irR : (float)(1.0 / kMinRho);
     // positive arguments: p >= 1e-14 and 1 / rho <= 1e14 (clamped above),
     // and 1 + (gamma+1)/(2 gamma) (p_rr / p - 1) > 1 under p_rr > p
-    const T cL = sqrt_pos(k.gamma_inv_eps * pL * icL);
-    const T cR = sqrt_pos(k.gamma_inv_eps * pR * icR);
-    T yL, yR, ipL, ipR;
-    root7_neg_z(pL, k, yL, ipL);
-    root7_neg_z(pR, k, yR, ipR);
-    const T base = (cL + cR - k.half_gm1 * (uR - uL)) * rcp_fast(cL * yL + cR * yR);
-    const T p_rr = pow7_inv_z(base, k);
-    const T qwL = (p_rr > pL) ? sqrt_pos(T(1) + k.gp1_2g * (p_rr * ipL - T(1))) : T(1);
-    const T qwR = (p_rr > pR) ? sqrt_pos(T(1) + k.gp1_2g * (p_rr * ipR - T(1))) : T(1);
-    const T SL = uL - cL * qwL;
-    const T SR = uR + cR * qwR;
-    const T dL = SL - uL, dR = SR - uR;
-    const T denom = rhoL * dL - rhoR * dR;
-    const T Ss_raw = ((pR - pL) * k.inv_eps + rhoL * uL * dL - rhoR * uR * dR) * rcp_fast(denom);
-    const T Ss = (denom != T(0)) ? Ss_raw : T(0);
+    const float cL = sqrt_fast(k.gamma_inv_eps * pL * icL);
+    const float cR = sqrt_fast(k.gamma_inv_eps * pR * icR);
+    float yL, yR, ipL, ipR;
+    root7_neg_z_f32(pL, k, yL, ipL);
+    root7_neg_z_f32(pR, k, yR, ipR);
+    const float base = (cL + cR - k.half_gm1 * (uR - uL)) * rcp_fast(cL * yL + cR * yR);
+    const float p_rr = ex2_fast(k.inv_z * lg2_fast(base));  // NaN for a negative base, as the reference's pow
+    const float qwL = (p_rr > pL) ? sqrt_fast(1.0f + k.gp1_2g * (p_rr * ipL - 1.0f)) : 1.0f;
+    const float qwR = (p_rr > pR) ? sqrt_fast(1.0f + k.gp1_2g * (p_rr * ipR - 1.0f)) : 1.0f;
+    const float SL = uL - cL * qwL;
+    const float SR = uR + cR * qwR;
+    const float dL = SL - uL, dR = SR - uR;
+    const float denom = rhoL * dL - rhoR * dR;
+    const float Ss_raw = ((pR - pL) * k.inv_eps + rhoL * uL * dL - rhoR * uR * dR) * rcp_fast(denom);
+    const float Ss = (denom != 0.0f) ? Ss_raw : 0.0f;
 
-    const bool useL = (SL >= T(0)) || (Ss >= T(0));
-    const bool star = useL ? (SL < T(0)) : (SR >= T(0));
-    T UK[NC], qK[NC];
+    const bool useL = (SL >= 0.0f) || (Ss >= 0.0f);
+    const bool star = useL ? (SL < 0.0f) : (SR >= 0.0f);
+    float UK[NC], qK[NC];
 #pragma unroll
     for (int n = 0; n < NC; ++n) {
         UK[n] = useL ? L[n] : R[n];
         qK[n] = useL ? qL[n] : qR[n];
     }
-    const T irK = useL ? irL : irR;
-    const T SK = useL ? SL : SR;
-    phys_flux<T, D, DIR>(UK, qK, k, F);
+    const float irK = useL ? irL : irR;
+    const float SK = useL ? SL : SR;
+    phys_flux<float, D, DIR>(UK, qK, k, F);
     // star state (HLLC.H:311-337): with m = rho_K (S_K - u_K), b = S_K - S*,
     // scale = m / b = m^2 / (m b) and p_K / m = p_K b / (m b)
-    const T rhoK = qK[0], uK = qK[1 + DIR], pK = qK[1 + D];
-    const T m = rhoK * (SK - uK);
-    const T bq = SK - Ss;
-    const T rmb = rcp_fast(m * bq);
-    const T scale = m * m * rmb;
-    const T eterm = UK[1 + D] * irK + (Ss - uK) * (Ss * k.eps + pK * bq * rmb);
+    const float rhoK = qK[0], uK = qK[1 + DIR], pK = qK[1 + D];
+    const float m = rhoK * (SK - uK);
+    const float bq = SK - Ss;
+    const float rmb = rcp_fast(m * bq);
+    const float scale = m * m * rmb;
+    const float eterm = UK[1 + D] * irK + (Ss - uK) * (Ss * k.eps + pK * bq * rmb);
     F[0] = star ? F[0] + SK * (scale - UK[0]) : F[0];
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-        const T s = (d == DIR) ? Ss : qK[1 + d];
+        const float s = (d == DIR) ? Ss : qK[1 + d];
         F[1 + d] = star ? F[1 + d] + SK * (s * scale - UK[1 + d]) : F[1 + d];
     }
     F[1 + D] = star ? F[1 + D] + SK * (eterm * scale - UK[1 + D]) : F[1 + D];
 }
 
-template <typename T, int D>
-__device__ __forceinline__ T wave_speed_fast(const T (&U)[D + 2], const K<T>& k)
+template <int D>
+__device__ __forceinline__ float wave_speed_f32(const float (&U)[D + 2], const K<float>& k)
 {
-    T q[D + 2], ir;
-    to_prim_fast<T, D>(U, k, q, ir);
-    T vsq = q[1] * q[1];
+    float q[D + 2], ir;
+    to_prim_f32<D>(U, k, q, ir);
+    float vsq = q[1] * q[1];
 #pragma unroll
     for (int d = 1; d < D; ++d) vsq = vsq + q[1 + d] * q[1 + d];
-    return sqrt_any(k.gamma_inv_eps * q[1 + D] * ir) + sqrt_any(vsq);
+    return sqrt_fast(k.gamma_inv_eps * q[1 + D] * ir) + sqrt_fast(vsq);
 }
 
 // Method dispatch: cell stage (reconstruction + half step for MUSCL-Hancock
@@ -628,7 +781,9 @@ struct Scheme {
                                                 const K<T>& k, T hdtdx, T (&UL)[NC], T (&UR)[NC])
     {
         if constexpr (kFast) {
-            muscl_cell_fast<T, D, DIR, (LIM < 0 ? 0 : LIM)>(Um, U0, Up, k, hdtdx, UL, UR);
+            constexpr int L = LIM < 0 ? 0 : LIM;
+            if constexpr (sizeof(T) == 8) muscl_cell_f64<D, DIR, L>(Um, U0, Up, k, hdtdx, UL, UR);
+            else muscl_cell_f32<D, DIR, L>(Um, U0, Up, k, hdtdx, UL, UR);
         } else if constexpr (kReconstruct) {
             muscl_cell<T, D, DIR>(Um, U0, Up, k, hdtdx, UL, UR);
         } else {
@@ -642,7 +797,8 @@ struct Scheme {
                                                 T dt_2dx, T (&F)[NC])
     {
         if constexpr (kFast) {
-            hllc_face_fast<T, D, DIR>(L, R, k, F);
+            if constexpr (sizeof(T) == 8) hllc_face_f64<D, DIR>(L, R, k, F);
+            else hllc_face_f32<D, DIR>(L, R, k, F);
         } else if constexpr (METHOD == M_MUSCL || METHOD == M_HLLC) {
             hllc_face<T, D, DIR>(L, R, k, F);
         } else if constexpr (METHOD == M_SLIC || METHOD == M_FORCE) {
@@ -654,8 +810,9 @@ struct Scheme {
 
     __device__ __forceinline__ static T speed(const T (&U)[NC], const K<T>& k)
     {
-        if constexpr (kFast) return wave_speed_fast<T, D>(U, k);
-        else return wave_speed<T, D>(U, k);
+        if constexpr (!kFast) return wave_speed<T, D>(U, k);
+        else if constexpr (sizeof(T) == 8) return wave_speed_f64<D>(U, k);
+        else return wave_speed_f32<D>(U, k);
     }
 };
 

@@ -238,7 +238,7 @@ __global__ void pack_slab_kernel(int NC, const FabDev f, const PackBox box, cons
 
 // ---------------------------------------------------------------- max speed
 // max_wave_speed (Source/System/Euler/Euler.cpp:46-74) over valid cells.
-template <typename T, int D>
+template <typename T, int D, bool FAST>
 __global__ void max_ws_kernel(const FabDev* __restrict__ fabs, const PackBox* __restrict__ boxes, int nboxes,
                               long long total, const Consts kc, unsigned long long* ws_bits, const StepScalars* scal)
 {
@@ -266,7 +266,9 @@ __global__ void max_ws_kernel(const FabDev* __restrict__ fabs, const PackBox* __
 #pragma unroll
             for (int u = 0; u < kWalkUnroll; ++u) {
                 if (c0 + 32 * u >= last) break;
-                const double s = (double)wave_speed<T, D>(U[u], k);
+                double s;
+                if constexpr (FAST) s = wave_speed_f64<D>(U[u], k);
+                else s = (double)wave_speed<T, D>(U[u], k);
                 wmax = fmax(wmax, s);
                 nan_seen = nan_seen || (s != s);
             }
@@ -275,6 +277,7 @@ __global__ void max_ws_kernel(const FabDev* __restrict__ fabs, const PackBox* __
     __syncwarp();
     for (int off = 16; off > 0; off >>= 1) wmax = fmax(wmax, __shfl_xor_sync(0xffffffffu, wmax, off));
     const bool any_nan = __any_sync(0xffffffffu, nan_seen);
+    if (FAST && wmax < 1e-140) wmax = 0.0;  // wave_speed_f64's offset of a state without pressure and motion
     if ((threadIdx.x & 31) == 0) {
         if (any_nan) atomicMax(ws_bits, 0x7ff8000000000000ull);
         else if (wmax > 0.0) atomicMax(ws_bits, (unsigned long long)__double_as_longlong(wmax));
@@ -492,27 +495,28 @@ cudaError_t launch_pack(int NC, bool fp32, const FabDev* fabs, const PackBox* bo
     }
 }
 
-template <typename T>
+template <typename T, bool FAST>
 static cudaError_t max_ws_dispatch(int D, const FabDev* fabs, const PackBox* boxes, int nboxes, long long total_cells,
                                    const Consts& k, unsigned long long* ws_bits, const StepScalars* scal,
                                    cudaStream_t s)
 {
     const int g = grid_for(total_cells, 4);
     switch (D) {
-    case 1: max_ws_kernel<T, 1><<<g, kThreads, 0, s>>>(fabs, boxes, nboxes, total_cells, k, ws_bits, scal); break;
-    case 2: max_ws_kernel<T, 2><<<g, kThreads, 0, s>>>(fabs, boxes, nboxes, total_cells, k, ws_bits, scal); break;
-    case 3: max_ws_kernel<T, 3><<<g, kThreads, 0, s>>>(fabs, boxes, nboxes, total_cells, k, ws_bits, scal); break;
+    case 1: max_ws_kernel<T, 1, FAST><<<g, kThreads, 0, s>>>(fabs, boxes, nboxes, total_cells, k, ws_bits, scal); break;
+    case 2: max_ws_kernel<T, 2, FAST><<<g, kThreads, 0, s>>>(fabs, boxes, nboxes, total_cells, k, ws_bits, scal); break;
+    case 3: max_ws_kernel<T, 3, FAST><<<g, kThreads, 0, s>>>(fabs, boxes, nboxes, total_cells, k, ws_bits, scal); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
 }
 
-cudaError_t launch_max_wave_speed(int D, bool fp32, const FabDev* fabs, const PackBox* boxes, int nboxes,
+cudaError_t launch_max_wave_speed(int D, bool fp32, bool fast, const FabDev* fabs, const PackBox* boxes, int nboxes,
                                   long long total_cells, const Consts& k, unsigned long long* ws_bits,
                                   const StepScalars* scal, cudaStream_t s)
 {
-    if (fp32) return max_ws_dispatch<float>(D, fabs, boxes, nboxes, total_cells, k, ws_bits, scal, s);
-    return max_ws_dispatch<double>(D, fabs, boxes, nboxes, total_cells, k, ws_bits, scal, s);
+    if (fp32) return max_ws_dispatch<float, false>(D, fabs, boxes, nboxes, total_cells, k, ws_bits, scal, s);
+    return fast ? max_ws_dispatch<double, true>(D, fabs, boxes, nboxes, total_cells, k, ws_bits, scal, s)
+                : max_ws_dispatch<double, false>(D, fabs, boxes, nboxes, total_cells, k, ws_bits, scal, s);
 }
 
 cudaError_t launch_box_sums(int NC, bool fp32, const FabDev* fabs, const PackBox* boxes, int nboxes, double* sums,

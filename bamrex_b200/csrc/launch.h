@@ -89,6 +89,11 @@ long long sweep_resident_warps(int D, int dir, int method, bool fp32, const Cons
 // The fast-path limiter for this configuration (MUSCL-Hancock, energy
 // limiting, gamma with 1/z = 7), or -1 for the general kernels.
 int fast_limiter(int D, int method, const Consts& k);
+// Whether a level may ask for the TMA-staged kernels: the fast path's
+// configurations, and a gamma that misses 1/z = 7 by more than its own
+// rounding but by less than 1e-12, for which the request runs the general
+// register kernels.
+bool tma_requestable(int D, int method, const Consts& k);
 
 // TMA-staged sweeps: the per-warp march (sweep_tma.cuh) and the block
 // wavefront (sweep_wave.cuh, wave = true), for the fast path in 2D and 3D.
@@ -117,7 +122,9 @@ cudaError_t launch_pack_slab(int NC, bool fp32, const FabDev& fab, const PackBox
 cudaError_t launch_pack(int NC, bool fp32, const FabDev* fabs, const PackBox* boxes, int nboxes,
                         long long total_cells, double* packed, int to_packed, cudaStream_t s);
 
-cudaError_t launch_max_wave_speed(int D, bool fp32, const FabDev* fabs, const PackBox* boxes, int nboxes,
+// fast (FP64): |u| + c as the fast path's sweeps form it, so that this
+// maximum and the one a sweep reduces are the same bits.
+cudaError_t launch_max_wave_speed(int D, bool fp32, bool fast, const FabDev* fabs, const PackBox* boxes, int nboxes,
                                   long long total_cells, const Consts& k, unsigned long long* ws_bits,
                                   const StepScalars* scal, cudaStream_t s);
 

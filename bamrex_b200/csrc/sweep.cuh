@@ -119,25 +119,42 @@ __device__ __forceinline__ void shfl_carry(const T (&cur)[NC], const T (&prev)[N
         out[n] = __shfl_sync(0xffffffffu, from_prev ? prev[n] : cur[n], (lane + 32 - shift) & 31);
 }
 
+// The running maximum of the wave speed |u| + c of a thread's updated cells,
+// in the kernel's own type, without a branch: the value by one comparison,
+// and the largest exponent field beside it (NaN and infinity show there; the
+// comparison alone would drop a NaN).
+template <typename T>
+struct WsMax {
+    T v = T(0);
+    int top = 0;
+    __device__ __forceinline__ static int bits(double w) { return __double2hiint(w) & 0x7fffffff; }
+    __device__ __forceinline__ static int bits(float w) { return __float_as_int(w) & 0x7fffffff; }
+    __device__ __forceinline__ void add(T w, bool counts)
+    {
+        w = counts ? w : T(0);
+        v = w > v ? w : v;
+        top = max(top, bits(w));
+    }
+    __device__ __forceinline__ bool bad() const { return top >= (sizeof(T) == 8 ? 0x7ff00000 : 0x7f800000); }
+};
+
 // Warp max of the wave speed, then one atomicMax per warp on the ordered bit
-// pattern (non-negative doubles order like their bits).  A NaN anywhere is
-// reported as the NaN bit pattern, which is larger than every finite value,
-// so the time step becomes NaN and the host sees BAMREX_ERR_NAN.
-__device__ __forceinline__ void reduce_ws(double ws, bool nan_seen, unsigned long long* dst)
+// pattern (non-negative doubles order like their bits).  A NaN or infinity
+// anywhere is reported as the NaN bit pattern, which is larger than every
+// finite value, so the time step becomes NaN and the host sees
+// BAMREX_ERR_NAN.
+template <typename T>
+__device__ __forceinline__ void reduce_ws(const WsMax<T>& w, unsigned long long* dst)
 {
+    double ws = (double)w.v;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) ws = fmax(ws, __shfl_xor_sync(0xffffffffu, ws, off));
-    const bool any_nan = __any_sync(0xffffffffu, nan_seen);
+    const bool any_bad = __any_sync(0xffffffffu, w.bad());
+    if (ws < 1e-140) ws = 0.0;  // wave_speed_f64's offset of a state without pressure and motion
     if ((threadIdx.x & 31) == 0) {
-        if (any_nan) atomicMax(dst, 0x7ff8000000000000ull);
+        if (any_bad) atomicMax(dst, 0x7ff8000000000000ull);
         else if (ws > 0.0) atomicMax(dst, (unsigned long long)__double_as_longlong(ws));
     }
-}
-
-__device__ __forceinline__ void track_ws(double w, double& wsmax, bool& nan_seen)
-{
-    wsmax = fmax(wsmax, w);
-    nan_seen = nan_seen || (w != w);
 }
 
 // ------------------------------------------------------------------ x sweep
@@ -155,8 +172,7 @@ __global__ void __launch_bounds__(kSweepThreads, min_blocks<T>()) sweep_x_kernel
     const int lane = threadIdx.x & 31;
     const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    double wsmax = 0.0;
-    bool nan_seen = false;
+    WsMax<T> wsmax;
 
     for (long long it = gw; it < a.total_items; it += nw) {
         const int b = a.boxes ? find_box(a.boxes, a.nboxes, it) : 0;
@@ -233,10 +249,7 @@ __global__ void __launch_bounds__(kSweepThreads, min_blocks<T>()) sweep_x_kernel
 #pragma unroll
                 for (int n = 0; n < NC; ++n) out[o + n * ons] = Un[n];
             }
-            if (ws_on) {
-                const double w = (double)S::speed(Un, k);
-                track_ws(upd ? w : 0.0, wsmax, nan_seen);
-            }
+            if (ws_on) wsmax.add(S::speed(Un, k), upd);
             if (fl) {
                 const int fo = o + 1;
                 if (fo >= s0 && (fo < s1 || (fo == s1 && last_seg))) {
@@ -252,7 +265,7 @@ __global__ void __launch_bounds__(kSweepThreads, min_blocks<T>()) sweep_x_kernel
             copy_state(Um2, Um2p);
         }
     }
-    if (a.ws_max) reduce_ws(wsmax, nan_seen, a.ws_max);
+    if (a.ws_max) reduce_ws(wsmax, a.ws_max);
 }
 
 // ----------------------------------------------------- marching sweeps
@@ -275,8 +288,7 @@ __global__ void __launch_bounds__(kSweepThreads, min_blocks<T>()) sweep_s_kernel
     const int lane = threadIdx.x & 31;
     const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    double wsmax = 0.0;
-    bool nan_seen = false;
+    WsMax<T> wsmax;
 
     for (long long it = gw; it < a.total_items; it += nw) {
         const int b = a.boxes ? find_box(a.boxes, a.nboxes, it) : 0;
@@ -502,10 +514,7 @@ __global__ void __launch_bounds__(kSweepThreads, min_blocks<T>()) sweep_s_kernel
 #pragma unroll
                 for (int n = 0; n < NC; ++n) po[n * ons] = Un[n];
             }
-            if (ws_on) {
-                const double w = (double)S::speed(Un, k);
-                track_ws(upd ? w : 0.0, wsmax, nan_seen);
-            }
+            if (ws_on) wsmax.add(S::speed(Un, k), upd);
             if (fl && active) {
                 const int fo = o + 1;
                 if (fo >= s0 && (fo < s1 || (fo == s1 && last_seg))) {
@@ -524,7 +533,7 @@ __global__ void __launch_bounds__(kSweepThreads, min_blocks<T>()) sweep_s_kernel
         }
     }
     if constexpr (DIR == 0) cp_async_wait_all();  // no copy outlives the kernel
-    if (a.ws_max) reduce_ws(wsmax, nan_seen, a.ws_max);
+    if (a.ws_max) reduce_ws(wsmax, a.ws_max);
 }
 
 }  // namespace bamrex

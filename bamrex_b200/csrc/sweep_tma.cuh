@@ -21,14 +21,14 @@
 // one per lane, fall into different banks).
 //
 // March.  Step q (the newest position loaded) does, for every lane: load
-// U(q); face q-2 (HLLC between the half-stepped states UR(q-3), UL(q-2) of
-// earlier steps); update of cell q-3 from faces q-3 and q-2; cell stage of
-// cell q-1 (limiter + half step from U(q-2), U(q-1), U(q)).  The face and
-// the cell stage of a step are independent instruction streams.  Register
-// slots rotate with the step index within the stage (S is a multiple of 4),
-// so the unrolled stage needs no register moves.  Positions run from
-// s0 - 2 to s1 + 2 (the last without a load); updates are stored for
-// s0 <= q - 3 < s1.
+// U(q); cell stage of cell q-1 (limiter + half step from U(q-2), U(q-1),
+// U(q)); face q-1 (HLLC between the half-stepped states UR(q-2) and UL(q-1));
+// update of cell q-2 from faces q-2 and q-1.  Between steps a lane keeps
+// U(q), U(q-1), UR(q-1) and the face flux q-1.  The steps of a stage are
+// unrolled without a branch between them (positions past the segment are
+// computed and not stored; stores are predicated), so a later step's cell
+// stage fills the waits of an earlier step's face.  Positions run from s0 - 2
+// to s1 + 1; updates are stored for s0 <= q - 2 < s1.
 #pragma once
 
 #include "common.cuh"
@@ -73,12 +73,17 @@ constexpr int tma_smem_bytes()
     return 1024 + kTmaWarps * TmaShape<T, D, DIR>::kWarpBytes + kTmaWarps * TmaShape<T, D, DIR>::NST * 8;
 }
 
-// Resident 128-thread blocks per SM the kernels are compiled for.
+// Resident 128-thread blocks per SM the kernels are compiled for.  The sweep
+// is bound by the FP64 pipe (two cycles per warp instruction, eight to the
+// result), and one thread's independent instructions fill it better than
+// more warps do: with 2 blocks (up to 255 registers) the compiler overlaps
+// the four steps of a stage.  4096^2 FP64 y sweep: 4 blocks 372 us, 3 blocks
+// 342 us, 2 blocks 307 us; FP32 storage 4 blocks 152 us, 3 blocks 149 us.
 #ifndef BAMREX_TMA_MIN_BLOCKS
-#define BAMREX_TMA_MIN_BLOCKS 3
+#define BAMREX_TMA_MIN_BLOCKS 2
 #endif
 #ifndef BAMREX_TMA_MIN_BLOCKS_F32
-#define BAMREX_TMA_MIN_BLOCKS_F32 4
+#define BAMREX_TMA_MIN_BLOCKS_F32 3
 #endif
 template <typename T>
 constexpr int tma_min_blocks() { return sizeof(T) == 4 ? BAMREX_TMA_MIN_BLOCKS_F32 : BAMREX_TMA_MIN_BLOCKS; }
@@ -92,7 +97,6 @@ __global__ void __launch_bounds__(kTmaThreads, tma_min_blocks<T>()) sweep_tma_ke
     constexpr int S = Sh::S;
     constexpr int NST = Sh::NST;
     constexpr int A = tma_dir_a(DIR), B_ = tma_dir_b(DIR);
-    static_assert(S % 4 == 0, "register slots rotate with period 4");
     static_assert(Sh::kSpan == 32 || Sh::kSpan == 64 || Sh::kSpan == 128, "x-sweep swizzle span");
 
     StepFactors<T> f;
@@ -117,8 +121,7 @@ __global__ void __launch_bounds__(kTmaThreads, tma_min_blocks<T>()) sweep_tma_ke
 
     const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    double wsmax = 0.0;
-    bool nan_seen = false;
+    WsMax<T> wsmax;
     bool failed = false;
 
     // x sweep: the XOR of this lane's line in the swizzled stage (the TMA
@@ -147,7 +150,7 @@ __global__ void __launch_bounds__(kTmaThreads, tma_min_blocks<T>()) sweep_tma_ke
         constexpr int q16 = 16 / (int)sizeof(T);
         const int pad = DIR == 0 ? ((s0 - 2 - Bx.lo[0]) & (q16 - 1)) : 0;
         const int P0 = s0 - 2 - pad;
-        const int Pend = s1 + 2;
+        const int Pend = s1 + 1;
         const int nstage = (Pend - P0) / S + 1;
         const void* tmap = Bx.tmap;
 
@@ -238,16 +241,13 @@ __global__ void __launch_bounds__(kTmaThreads, tma_min_blocks<T>()) sweep_tma_ke
         };
         int flushed = -1;  // x sweep: out-stages written out so far
 
-        T U[4][NC], UL[2][NC], UR[2][NC], F[2][NC];
+        // U(q-1), U(q-2), UR(q-2) and the face flux q-2 of the step before
+        T U1[NC], U2[NC], URm[NC], Fm[NC];
+        benign(U1);
+        benign(U2);
+        benign(URm);
 #pragma unroll
-        for (int s = 0; s < 4; ++s) benign(U[s]);
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-            benign(UL[s]);
-            benign(UR[s]);
-#pragma unroll
-            for (int n = 0; n < NC; ++n) F[s][n] = T(0);
-        }
+        for (int n = 0; n < NC; ++n) Fm[n] = T(0);
 
         int st_fail = -1;
         for (int st = 0; st < nstage; ++st) {
@@ -261,48 +261,51 @@ __global__ void __launch_bounds__(kTmaThreads, tma_min_blocks<T>()) sweep_tma_ke
             phase ^= 1u << buf;
             const unsigned char* sb = wbuf_p + buf * Sh::kStageBytes;
             const int qbase = P0 + st * S;
-            T* orow = ocol + (long long)(qbase - 3) * ostep;
+            T* orow = ocol + (long long)(qbase - 2) * ostep;
 #pragma unroll
             for (int j = 0; j < S; ++j) {
                 const int q = qbase + j;
-                if (q > Pend) break;
-                // U(q) -> slot j % 4 (U(q-1): (j+3)%4, U(q-2): (j+2)%4, U(q-3): (j+1)%4)
+                T U0[NC];
 #pragma unroll
-                for (int n = 0; n < NC; ++n) U[j % 4][n] = elem(sb, n, j);
-                // face q-2 from UR(q-3) (slot (j+1)%2) and UL(q-2) (slot j%2)
-                T Fn[NC];
-                Sc::face(UR[(j + 1) % 2], UL[j % 2], k, f.half_dx_dt, f.dt_2dx, Fn);
-                // update of cell q-3 from faces q-3 (slot (j+1)%2) and q-2
+                for (int n = 0; n < NC; ++n) U0[n] = elem(sb, n, j);
+                // cell q-1, then the face between q-2 and q-1
+                T UL[NC], UR[NC], Fn[NC];
+                Sc::cell(U2, U1, U0, k, f.hdtdx, UL, UR);
+                Sc::face(URm, UL, k, f.half_dx_dt, f.dt_2dx, Fn);
+                // update of cell q-2 from faces q-2 and q-1
                 T Un[NC];
 #pragma unroll
-                for (int n = 0; n < NC; ++n) Un[n] = U[(j + 1) % 4][n] - f.dtdx * (Fn[n] - F[(j + 1) % 2][n]);
-                const int o = q - 3;
+                for (int n = 0; n < NC; ++n) Un[n] = fma(-f.dtdx, Fn[n] - Fm[n], U2[n]);
+                const int o = q - 2;
                 const bool upd = active && o >= s0 && o < s1;
                 if constexpr (DIR == 0) {
-                    // position o is slot (j + S - 3) % S of out-stage st (j >= 3)
-                    // or st - 1 (j < 3); that one is complete after step 2
-                    const int pj = (j + S - 3) % S;
+                    // position o is slot (j + S - 2) % S of out-stage st (j >= 2)
+                    // or st - 1 (j < 2); that one is complete after step 1
+                    const int pj = (j + S - 2) % S;
 #pragma unroll
                     for (int n = 0; n < NC; ++n)
                         *reinterpret_cast<T*>(osb + (n * 32 + lane) * kSpan + (((uint32_t)(pj * (int)sizeof(T))) ^ xl)) =
                             Un[n];
-                    if (j == 2 && st >= 1) {
+                    if (j == 1 && st >= 1) {
                         flush(st - 1);
                         flushed = st - 1;
                     }
-                } else if (upd) {
+                } else {
                     T* po = orow + (long long)j * ostep;
 #pragma unroll
-                    for (int n = 0; n < NC; ++n) po[n * ons] = Un[n];
+                    for (int n = 0; n < NC; ++n) st_global_if(po + n * ons, Un[n], upd);
                 }
-                if constexpr (WS) {
-                    const double w = (double)Sc::speed(Un, k);
-                    track_ws(upd ? w : 0.0, wsmax, nan_seen);
+                if constexpr (WS) wsmax.add(Sc::speed(Un, k), upd);
+#pragma unroll
+                for (int n = 0; n < NC; ++n) {
+                    Fm[n] = Fn[n];
+                    URm[n] = UR[n];
                 }
 #pragma unroll
-                for (int n = 0; n < NC; ++n) F[j % 2][n] = Fn[n];
-                // cell stage of cell q-1 -> slot (j+1)%2
-                Sc::cell(U[(j + 2) % 4], U[(j + 3) % 4], U[j % 4], k, f.hdtdx, UL[(j + 1) % 2], UR[(j + 1) % 2]);
+                for (int n = 0; n < NC; ++n) {
+                    U2[n] = U1[n];
+                    U1[n] = U0[n];
+                }
             }
             // every lane is done with this buffer: refill it with stage st + NST
             __syncwarp();
@@ -328,7 +331,7 @@ __global__ void __launch_bounds__(kTmaThreads, tma_min_blocks<T>()) sweep_tma_ke
         }
     }
     if constexpr (WS) {
-        if (!failed) reduce_ws(wsmax, nan_seen, a.ws_max);
+        if (!failed) reduce_ws(wsmax, a.ws_max);
     }
 }
 

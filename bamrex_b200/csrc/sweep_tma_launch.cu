@@ -50,6 +50,15 @@ int smem_bytes(int D, int dir, bool fp32, bool wave)
     return dir == 0 ? smem_bytes_t<3, 0>(fp32, wave) : dir == 1 ? smem_bytes_t<3, 1>(fp32, wave) : smem_bytes_t<3, 2>(fp32, wave);
 }
 
+template <int D, int DIR>
+int stage_positions_t(bool fp32) { return fp32 ? TmaShape<float, D, DIR>::S : TmaShape<double, D, DIR>::S; }
+
+int stage_positions(int D, int dir, bool fp32)
+{
+    if (D == 2) return dir == 0 ? stage_positions_t<2, 0>(fp32) : stage_positions_t<2, 1>(fp32);
+    return dir == 0 ? stage_positions_t<3, 0>(fp32) : dir == 1 ? stage_positions_t<3, 1>(fp32) : stage_positions_t<3, 2>(fp32);
+}
+
 const void* pick(int D, int dir, bool fp32, int lim, bool ws, bool wave)
 {
     return fp32 ? pick_tma_kernel<float>(D, dir, lim, ws, wave) : pick_tma_kernel<double>(D, dir, lim, ws, wave);
@@ -87,7 +96,7 @@ cudaError_t encode_sweep_tmap(void* out, bool fp32, int D, int NC, int dir, bool
     if (!fn) return cudaErrorNotSupported;
     const int es = fp32 ? 4 : 8;
     // positions per tile along dir, lines across it
-    const int S = wave ? tma_pass_positions(true, dir) : (fp32 ? TmaShape<float, 2, 1>::S : TmaShape<double, 2, 1>::S);
+    const int S = wave ? tma_pass_positions(true, dir) : stage_positions(D, dir, fp32);
     const int NL = tma_item_lines(wave, dir);
     const int wb = NL / wa;
     cuuint64_t dims[4], strides[3];

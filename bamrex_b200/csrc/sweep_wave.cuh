@@ -101,8 +101,7 @@ __global__ void __launch_bounds__(kWaveThreads, wave_min_blocks<T>()) sweep_wave
     }
     __syncthreads();
     uint32_t phase = 0;
-    double wsmax = 0.0;
-    bool nan_seen = false;
+    WsMax<T> wsmax;
     bool failed = false;
 
     // ring slot s of component n for this thread's line
@@ -236,10 +235,7 @@ __global__ void __launch_bounds__(kWaveThreads, wave_min_blocks<T>()) sweep_wave
             T* po = ocol + (long long)c * ostep;
 #pragma unroll
             for (int n = 0; n < NC; ++n) st_global_if(po + n * ons, Un[n], upd);
-            if constexpr (WS) {
-                const double w = (double)Sc::speed(Un, k);
-                track_ws(upd ? w : 0.0, wsmax, nan_seen);
-            }
+            if constexpr (WS) wsmax.add(Sc::speed(Un, k), upd);
         }
         if (failed) {
             // let every stage still in flight land (each wait bounded):
@@ -255,7 +251,7 @@ __global__ void __launch_bounds__(kWaveThreads, wave_min_blocks<T>()) sweep_wave
         }
     }
     if constexpr (WS) {
-        if (!failed) reduce_ws(wsmax, nan_seen, a.ws_max);
+        if (!failed) reduce_ws(wsmax, a.ws_max);
     }
 }
 
