@@ -155,81 +155,81 @@ bool overlaps(const bamrex_array4& a, const bamrex_array4& b, int NC)
     return ra.first < rb.second && rb.first < ra.second;
 }
 
-// Work items of one box in one sweep direction.
-// Work items of one box for the sweep of direction dir: warp-per-row-segment
-// items for the x sweep (march = false), else segments of 32 adjacent
-// columns (rows for the marching x sweep).
-// The box's segments have equal lengths (at most seglen; multiples of 32
-// for the row kernel), returned in box_seglen.
+// Work items of one box for the sweep of direction dir by the register
+// kernels: chunks of row groups for the x sweep (march = false; row_p
+// positions per group, ngroup groups per row), else segments of 32 adjacent
+// columns (rows for the marching x sweep).  The box's segments have equal
+// lengths (at most seglen), returned in box_seglen.
 void box_items(int dir, const int* lo, const int* hi, int seglen, long long& items, int& nseg, int& ngroup,
-               bool march = false, int* box_seglen = nullptr)
+               bool march = false, int* box_seglen = nullptr, int row_p = 4)
 {
     const int n[3] = { hi[0] - lo[0] + 1, hi[1] - lo[1] + 1, hi[2] - lo[2] + 1 };
-    nseg = (n[dir] + seglen - 1) / seglen;
-    int bl = (n[dir] + nseg - 1) / nseg;
-    if (dir == 0 && !march) bl = std::min(seglen, (bl + 31) / 32 * 32);
-    if (box_seglen) *box_seglen = bl;
     if (dir == 0 && !march) {
-        ngroup = 1;
-        items = (long long)n[1] * n[2] * nseg;
-    } else {
-        // 32 columns of the plane across dir per group (boxes narrower than
-        // 32 cells fill the lanes from the next plane)
-        const long long cols = (long long)(dir == 0 ? n[1] : n[0]) * (dir == 2 ? n[1] : n[2]);
-        ngroup = (int)((cols + 31) / 32);
-        items = (long long)ngroup * nseg;
+        nseg = 1;
+        if (box_seglen) *box_seglen = n[0];
+        ngroup = (n[0] + 4 + row_p - 1) / row_p;
+        items = ((long long)ngroup * n[1] * n[2] + kRowOwned - 1) / kRowOwned;
+        return;
     }
+    nseg = (n[dir] + seglen - 1) / seglen;
+    if (box_seglen) *box_seglen = (n[dir] + nseg - 1) / nseg;
+    // 32 columns of the plane across dir per group (boxes narrower than
+    // 32 cells fill the lanes from the next plane)
+    const long long cols = (long long)(dir == 0 ? n[1] : n[0]) * (dir == 2 ? n[1] : n[2]);
+    ngroup = (int)((cols + 31) / 32);
+    items = (long long)ngroup * nseg;
 }
 
-// Segment length: the longest that still gives every resident warp several
-// items (few partial waves); x segments of the row kernel are multiples of 32.
+// Segment length of a march: the one with the least estimated time, the
+// rounds in which the resident warps take the items times the mean steps of
+// an item (its cells and 5 more: warm-up and the first loads).  Small boxes
+// and levels get short segments, so that one round of them covers the chip
+// (one 64^3 box: y and z flux calls 80 us in 64-cell segments, 128 warps);
+// large ones long segments.
 int choose_seglen(int dir, const std::vector<bamrex_box>& boxes, long long resident_warps, bool march = false)
 {
-    static const int xs[] = { 2048, 1024, 512, 256, 128, 64, 32 };
-    static const int ss[] = { 256, 128, 96, 64, 48, 32, 24, 16 };
-    const bool rows = dir == 0 && !march;
-    const int* cand = rows ? xs : ss;
-    const int ncand = rows ? 7 : 8;
-    const long long want = std::max(1LL, resident_warps) * 6;
-    for (int c = 0; c < ncand; ++c) {
-        long long tot = 0;
-        int nseg, ngroup;
-        long long it;
+    std::vector<int> cand = { 256, 192, 128, 96, 64, 48, 32, 24, 16, 12, 8 };
+    int nmax = 1;
+    for (const auto& b : boxes) nmax = std::max(nmax, b.hi[dir] - b.lo[dir] + 1);
+    for (int m = 1; m <= 24; ++m)
+        if ((nmax + m - 1) / m >= 4) cand.push_back(std::min(256, (nmax + m - 1) / m));
+    const long long W = std::max(1LL, resident_warps);
+    int best = 64;
+    double best_time = -1;
+    for (int c : cand) {
+        long long items = 0, steps = 0;
         for (const auto& b : boxes) {
-            box_items(dir, b.lo, b.hi, cand[c], it, nseg, ngroup, march);
-            tot += it;
+            long long it;
+            int nseg, ngroup;
+            box_items(dir, b.lo, b.hi, c, it, nseg, ngroup, march);
+            items += it;
+            steps += (long long)ngroup * (b.hi[dir] - b.lo[dir] + 1 + 5LL * nseg);
         }
-        if (tot >= want) return cand[c];
+        const double t = (double)((items + W - 1) / W) * (double)steps / (double)items;
+        if (best_time < 0 || t < best_time) {
+            best = c;
+            best_time = t;
+        }
     }
-    return cand[ncand - 1];
+    return best;
 }
 
-// Lane-cell slots of the two x-sweep kernels over a set of boxes: the row
-// kernel spends two extra 32-cell chunks on every row segment (its
-// software pipeline), the marching kernel four extra cells per segment and
-// idle lanes in its last group of 32 rows; its per-cell cost
-// carries a 30% allowance for staging rows through shared memory (measured
-// on 4096^2 in boxes of 32 to 4096 cells).
-bool prefer_x_march(int D, const std::vector<bamrex_box>& boxes, int seg_rows, int seg_march)
+// Whether a level's rows are so short (24 cells or fewer on average) that the
+// marching x kernel serves it: a row of the row groups carries four halo
+// positions, and its halo lanes read the neighbours' rows.  3D 256^3, x sweep
+// by row groups / marching: FP64 in 64^3 boxes 566 / 650 us, 32^3 571 / 673,
+// 16^3 615 / 644, 8^3 894 / 850; FP32 32^3 300 / 433, 16^3 435 / 516, 240^3 in
+// 12^3 701 / 527.  The general path, whose face calls the power functions,
+// gains nothing from four cells per lane: rows up to 512 cells march.
+bool narrow_rows(const std::vector<bamrex_box>& boxes, bool fast)
 {
-    if (D < 2) return false;
-    double rows = 0, march = 0;
+    long long cells = 0, rows = 0;
     for (const auto& b : boxes) {
-        const long long n0 = b.hi[0] - b.lo[0] + 1, n1 = b.hi[1] - b.lo[1] + 1, n2 = b.hi[2] - b.lo[2] + 1;
-        long long items;
-        int nseg, ngroup, bl;
-        box_items(0, b.lo, b.hi, seg_rows, items, nseg, ngroup, false, &bl);
-        for (long long x = 0; x < n0; x += bl) {
-            const long long len = std::min<long long>(bl, n0 - x);
-            rows += (double)(n1 * n2) * 32.0 * (double)((len + 64 + 31) / 32);
-        }
-        box_items(0, b.lo, b.hi, seg_march, items, nseg, ngroup, true, &bl);
-        for (long long x = 0; x < n0; x += bl) {
-            const long long len = std::min<long long>(bl, n0 - x);
-            march += 1.3 * (double)((n1 * n2 + 31) / 32 * 32) * (double)(len + 4);
-        }
+        const long long r = (long long)(b.hi[1] - b.lo[1] + 1) * (b.hi[2] - b.lo[2] + 1);
+        rows += r;
+        cells += r * (b.hi[0] - b.lo[0] + 1);
     }
-    return march < rows;
+    return cells <= (fast ? 24 : 512) * rows;
 }
 
 // ---- TMA-staged sweeps (sweep_tma.cuh, sweep_wave.cuh): lane groups and
@@ -347,36 +347,31 @@ int choose_tma_seglen(int D, int dir, const std::vector<bamrex_box>& boxes, long
     return best;
 }
 
-// Kernel of a sweep direction when the level leaves the choice to the
-// library: the kind with the least estimated time, from the slot-steps each
-// spends on the level's boxes (idle lanes, warm-up, pass rounding included,
-// at the segment lengths each would choose) times a measured time per
-// slot-step (B200, 4096^2 2D and 256^3 3D, per direction and storage type;
-// the FP64 3D y / z march and TMA figures refitted on 256^3 levels in 16^3,
-// 32^3 and 64^3 boxes, where the TMA march was the fastest y / z kernel).
-// rows / march: the two L2-loading x kernels.
-int auto_sweep_kind(int D, int d, bool fp32, const std::vector<bamrex_box>& boxes, int seg_rows, int seg_march,
-                    int seg_tma, int seg_wave, bool allow_tma)
+// Kernel of a y / z sweep when the level leaves the choice to the library:
+// the kind with the least estimated time, from the slot-steps each spends on
+// the level's boxes (idle lanes, warm-up, pass rounding included, at the
+// segment lengths each would choose) times a measured time per slot-step
+// (B200, one box of 4096^2 in 2D and 256^3 in 3D, per direction and storage
+// type).  The x sweep is the register kernels' (row groups or march): they
+// are faster than the TMA-staged ones on every box size measured.
+int auto_sweep_kind(int D, int d, bool fp32, const std::vector<bamrex_box>& boxes, int seg_march, int seg_tma, int seg_wave)
 {
-    // picoseconds per slot-step: [fp32][D - 2][d] x {rows, march, TMA, wave}
-    static const double ps[2][2][3][4] = {
-        { { { 28, 37, 53, 27 }, { 0, 30, 29, 29 }, { 0, 0, 0, 0 } },
-          { { 39, 47, 70, 27.5 }, { 0, 31.5, 25, 28 }, { 0, 35, 27.5, 31 } } },
-        { { { 12.6, 16, 18.5, 13.5 }, { 0, 15, 11, 15 }, { 0, 0, 0, 0 } },
-          { { 16, 20, 23, 17 }, { 0, 19, 14, 19 }, { 0, 21, 15, 20 } } },
+    if (d == 0) return BAMREX_STAGING_REGISTERS;
+    // picoseconds per slot-step: [fp32][D - 2][d - 1] x {march, TMA, wave}
+    static const double ps[2][2][2][3] = {
+        { { { 22.6, 17.9, 23.8 }, { 0, 0, 0 } }, { { 24, 18.8, 25 }, { 26.2, 20.6, 26.5 } } },
+        { { { 14.1, 9.9, 13.4 }, { 0, 0, 0 } }, { { 14.4, 11.4, 16.7 }, { 15, 13, 18 } } },
     };
-    const double* c = ps[fp32 ? 1 : 0][D - 2][d];
-    double rows = 0, march = 0, tma = 0, wave = 0;
+    const double* c = ps[fp32 ? 1 : 0][D - 2][d - 1];
+    double march = 0, tma = 0, wave = 0;
     const int pw = tma_pass_positions(true, d), nlw = tma_item_lines(true, d);
     for (const auto& b : boxes) {
         const int n[3] = { b.hi[0] - b.lo[0] + 1, b.hi[1] - b.lo[1] + 1, b.hi[2] - b.lo[2] + 1 };
-        const int A = d == 0 ? 1 : 0, B = d == 2 ? 1 : 2;
-        const long long lines = (long long)n[A] * n[B];
+        const long long lines = (long long)n[0] * n[d == 1 ? 2 : 1];
         auto segs = [&](int seglen, auto&& per) {
             const int nseg = (n[d] + seglen - 1) / seglen, bl = (n[d] + nseg - 1) / nseg;
             for (int x = 0; x < n[d]; x += bl) per(std::min(bl, n[d] - x));
         };
-        if (d == 0) segs(seg_rows, [&](int len) { rows += (double)lines * 32.0 * ((len + 64 + 31) / 32); });
         segs(seg_march, [&](int len) { march += (double)((lines + 31) / 32 * 32) * (len + 4); });
         long long it;
         int nseg, ng, wa, bl;
@@ -385,13 +380,13 @@ int auto_sweep_kind(int D, int d, bool fp32, const std::vector<bamrex_box>& boxe
         tma_box_items(D, d, b.lo, b.hi, seg_wave, nlw, it, nseg, ng, wa, bl);
         segs(seg_wave, [&](int len) { wave += (double)ng * nlw * ((len + 3 + pw - 1) / pw + 1) * pw; });
     }
-    double best = d == 0 ? std::min(rows * c[0], march * c[1]) : march * c[1];
+    double best = march * c[0];
     int kind = BAMREX_STAGING_REGISTERS;
-    if (allow_tma && tma * c[2] < best) {
-        best = tma * c[2];
+    if (tma * c[1] < best) {
+        best = tma * c[1];
         kind = BAMREX_STAGING_TMA;
     }
-    if (allow_tma && wave * c[3] < best) kind = BAMREX_STAGING_WAVE;
+    if (wave * c[2] < best) kind = BAMREX_STAGING_WAVE;
     return kind;
 }
 
@@ -516,10 +511,15 @@ static int per_box_sweep(int method, int dir, int D, const bamrex_box* bx, const
     if (Uout) B.out = to_fab(*Uout);
     if (flux && flux->p) B.flux = to_fab(*flux);
     const std::vector<bamrex_box> one(1, *bx);
-    const bool march = dir == 0 && prefer_x_march(D, one, 512, 64);
-    a.seglen = (dir == 0 && !march) ? 512 : 64;
+    a.seglen = dir == 0 ? bx->hi[0] - bx->lo[0] + 1 : choose_seglen(dir, one, sweep_resident_warps(D, dir, method, false, k));
     long long items;
-    box_items(dir, B.lo, B.hi, a.seglen, items, B.nseg, B.ngroup, march, &B.seglen);
+    box_items(dir, B.lo, B.hi, a.seglen, items, B.nseg, B.ngroup, false, &B.seglen, row_positions(fast_limiter(D, method, k)));
+    // pairs of the row lie at an even distance from lo: aligned when cell lo
+    // and the strides are
+    auto paired = [&](const bamrex_array4& f) {
+        return ((uintptr_t)(f.p + (B.lo[0] - f.begin[0])) & 15) == 0 && !((f.jstride | f.kstride | f.nstride) & 1);
+    };
+    a.rows = paired(Uin) && (!Uout || paired(*Uout)) ? kRowsBoxPaired : kRowsBox;
     B.item_begin = 0;
     a.total_items = items;
     a.halo = H;
@@ -529,7 +529,7 @@ static int per_box_sweep(int method, int dir, int D, const bamrex_box* bx, const
     a.k = k;
     a.ws_max = nullptr;
     a.do_update = Uout ? 1 : 0;
-    BX_CK(launch_sweep(D, dir, method, false, a, (cudaStream_t)stream, march));
+    BX_CK(launch_sweep(D, dir, method, false, a, (cudaStream_t)stream));
     return BAMREX_OK;
 }
 
@@ -1081,36 +1081,30 @@ extern "C" int bamrex_level_create(bamrex_level** out, const bamrex_level_desc* 
         return m;
     };
     std::vector<SweepBox> sweep_host[3];
-    // x-sweep kernel: one warp per row segment, or one thread per row
-    // (levels of narrow boxes); automatic by the lane-slot estimate
-    if (desc->x_mode == BAMREX_XSWEEP_MARCH) L->x_march = D >= 2;
-    else if (desc->x_mode == BAMREX_XSWEEP_ROWS) L->x_march = false;
-    else {
-        const int sr = desc->x_segment > 0 ? (int)align_up((size_t)desc->x_segment, 32) : reg_seg(0, false);
-        const int sm = desc->x_segment > 0 ? desc->x_segment : reg_seg(0, true);
-        L->x_march = prefer_x_march(D, L->boxes, sr, sm);
-    }
+    // the register kernel of the x sweep when the caller leaves it open
+    L->x_march = D >= 2 && (desc->x_mode == BAMREX_XSWEEP_MARCH || (desc->x_mode == BAMREX_XSWEEP_AUTO && narrow_rows(L->boxes, fast_limiter(D, L->method, L->k) >= 0)));
+    const int row_p = row_positions(fast_limiter(D, L->method, L->k));
     for (int d = 0; d < D; ++d) {
         if (L->sweep_kind[d] >= 0) continue;
         if (!tma_supported(D, L->method, L->k)) {
             L->sweep_kind[d] = BAMREX_STAGING_REGISTERS;
             continue;
         }
-        auto seg_for = [&](bool tma_kind, bool wave, bool march) {
-            const int user = d == 0 ? desc->x_segment : desc->s_segment;
-            if (user > 0) return user;
-            return tma_kind ? tma_seg(d, wave) : reg_seg(d, march);
+        auto seg_for = [&](bool tma_kind, bool wave) {
+            if (d == 0) return 0;
+            if (desc->s_segment > 0) return desc->s_segment;
+            return tma_kind ? tma_seg(d, wave) : reg_seg(d, false);
         };
-        const int sr = d == 0 ? (int)align_up((size_t)seg_for(false, false, false), 32) : 0;
-        const int sm = seg_for(false, false, d == 0);
-        L->sweep_kind[d] = auto_sweep_kind(D, d, L->fp32, L->boxes, sr, sm, seg_for(true, false, false),
-                                           seg_for(true, true, false), true);
+        L->sweep_kind[d] = auto_sweep_kind(D, d, L->fp32, L->boxes, seg_for(false, false), seg_for(true, false),
+                                           seg_for(true, true));
     }
     for (int d = 0; d < D; ++d) {
         const bool march = d == 0 && L->x_march;
         L->seglen[d] = d == 0 ? desc->x_segment : desc->s_segment;
-        if (L->seglen[d] <= 0) L->seglen[d] = L->tma(d) ? tma_seg(d, L->wave(d)) : reg_seg(d, march);
-        if (d == 0 && !march && !L->tma(d)) L->seglen[d] = (int)align_up((size_t)L->seglen[d], 32);
+        if (L->seglen[d] <= 0) {
+            if (L->tma(d)) L->seglen[d] = tma_seg(d, L->wave(d));
+            else L->seglen[d] = d == 0 && !march ? L->domain.hi[0] - L->domain.lo[0] + 1 : reg_seg(d, march);
+        }
         long long acc = 0;
         for (int b = 0; b < nb; ++b) {
             SweepBox sb;
@@ -1125,7 +1119,7 @@ extern "C" int bamrex_level_create(bamrex_level** out, const bamrex_level_desc* 
                               sb.seglen);
                 sb.xoff = front;
             } else {
-                box_items(d, sb.lo, sb.hi, L->seglen[d], it, sb.nseg, sb.ngroup, march, &sb.seglen);
+                box_items(d, sb.lo, sb.hi, L->seglen[d], it, sb.nseg, sb.ngroup, march, &sb.seglen, row_p);
             }
             sb.item_begin = acc;
             acc += it;
@@ -1156,12 +1150,14 @@ extern "C" int bamrex_level_create(bamrex_level** out, const bamrex_level_desc* 
         }
     }
 
-    // ---- x halos read in place by the marching x sweep: per box and side,
-    // the same-level box that holds the box's whole x ghost slab (inside the
-    // domain); the step's x fill then leaves those slabs out
+    // ---- x halos read in place by the register kernels' x sweep: per box
+    // and side, the same-level box that holds the box's whole x ghost slab
+    // (inside the domain); the step's x fill then leaves those slabs out.
+    // The row groups read pairs of cells: both boxes' rows must pair the same
+    // way there (even distances between their low ends).
     std::vector<int> xnb[2];
     std::vector<GhostOp> ghost_x;
-    if (D >= 2 && L->x_march && !L->tma(0)) {
+    if (D >= 2 && !L->tma(0)) {
         for (int side = 0; side < 2; ++side) xnb[side].assign((size_t)nb, -1);
         std::vector<int> hits;
         int nfused = 0;
@@ -1181,6 +1177,8 @@ extern "C" int bamrex_level_create(bamrex_level** out, const bamrex_level_desc* 
                     const bamrex_box& Q = L->boxes[q];
                     bool in = q != b;
                     for (int e = 0; e < 3 && in; ++e) in = Q.lo[e] <= slab.lo[e] && slab.hi[e] <= Q.hi[e];
+                    const int first = side == 0 ? L->boxes[b].lo[0] : L->boxes[b].hi[0] + 1;
+                    in = in && (L->x_march || (((first - Q.lo[0]) | (first - L->boxes[b].lo[0])) & 1) == 0);
                     if (in) {
                         xnb[side][(size_t)b] = q;
                         ++nfused;
@@ -1676,7 +1674,8 @@ int host_step_enqueue(bamrex_level* L, const double* host_in, double* host_out, 
         sb.flux.p = nullptr;
         const bool march = dir == 0 && L->x_march;
         long long items;
-        box_items(dir, sb.lo, sb.hi, L->seglen[dir], items, sb.nseg, sb.ngroup, march, &sb.seglen);
+        box_items(dir, sb.lo, sb.hi, L->seglen[dir], items, sb.nseg, sb.ngroup, march, &sb.seglen,
+                  row_positions(fast_limiter(D, L->method, L->k)));
         sb.item_begin = 0;
         sa.total_items = items;
         sa.seglen = L->seglen[dir];

@@ -7,6 +7,14 @@ namespace bamrex {
 
 constexpr int kMaxComp = 8;
 
+// The x sweep by row groups (sweep_row.cuh): positions per lane (fast path /
+// general path) and the groups of a 32-lane chunk that store their cells.
+__host__ __device__ constexpr int row_group(int fast_lim) { return fast_lim >= 0 ? 4 : 2; }
+constexpr int kRowOwned = 30;
+// Whose fabs that sweep works on: a level's, or one box of a caller's whose
+// rows are aligned to pairs of elements or not.
+enum { kRowsLevel = 0, kRowsBoxPaired = 1, kRowsBox = 2 };
+
 // Per-run physical and limiter constants.  Everything derived from gamma is
 // computed on the host with the reference's own expressions
 // (Source/Fluxes/HLLC.H:269-280, Source/System/FluidSystem.cpp:73-101) so the
@@ -61,7 +69,7 @@ struct SweepBox {
     FabDev in, out, flux;      // flux.p == nullptr: no flux output
     long long item_begin;      // first work item of this box
     int nseg;                  // segments along the sweep direction
-    int ngroup;                // lane groups of 32 columns (marching sweeps)
+    int ngroup;                // lane groups of 32 columns (marching sweeps); row groups per row (x sweep)
     int seglen;                // cells per segment (the last one may be shorter)
     // TMA-staged sweeps (sweep_tma.cuh): the tensor map of `in` for this
     // direction (device memory), lines of a lane group along the faster
@@ -70,9 +78,9 @@ struct SweepBox {
     const void* tmap;
     int wa;
     int xoff;
-    // marching x sweep: the same-level fab holding all of this box's ghost
-    // cells below lo (xnb[0]) / above hi (xnb[1]) in x, read in place of
-    // the ghost cells when SweepArgs::xnb_on (p == nullptr: none)
+    // x sweep of the register kernels: the same-level fab holding all of this
+    // box's ghost cells below lo (xnb[0]) / above hi (xnb[1]) in x, read in
+    // place of the ghost cells when SweepArgs::xnb_on (p == nullptr: none)
     FabDev xnb[2];
 };
 
@@ -102,7 +110,8 @@ struct SweepArgs {
     unsigned long long* ws_max;  // non-null: reduce max wave speed of Uout
     int do_update;             // 0: flux-only mode
     int* status;
-    int xnb_on;                // marching x sweep: read x halos from SweepBox::xnb
+    int xnb_on;                // x sweep: read x halos from SweepBox::xnb
+    int rows;                  // x sweep by row groups: whose fabs (kRows*)
 };
 
 }  // namespace bamrex

@@ -76,9 +76,12 @@ struct UpdateArgs {
 
 int device_sm_count();
 
+// The x sweep by row groups (sweep_row.cuh): positions per lane (a row of n
+// cells is ceil((n + 4) / positions) groups; a chunk owns kRowOwned of them).
+inline int row_positions(int fast_lim) { return row_group(fast_lim); }
+
 // march: run the x sweep (dir 0, D >= 2) as one thread per row instead of
-// one warp per row segment; the box table's items must be laid out to match
-// (sweep_items).
+// by row groups; the box table's items must be laid out to match (box_items).
 cudaError_t launch_sweep(int D, int dir, int method, bool fp32, const SweepArgs& a, cudaStream_t s,
                          bool march = false);
 

@@ -7,15 +7,12 @@
 //
 // Work decomposition: a launch covers every box of a sweep (the device box
 // table); each warp takes work items from a grid-stride loop.
-//  * x sweep (contiguous direction): an item is a segment of one row.  The
-//    warp marches along the row in 32-cell chunks, lane t holding cell
-//    x0+t; neighbour states come from warp shuffles, and the values of
-//    earlier chunks carry the stencil across chunk boundaries.
+//  * x sweep (contiguous direction): row groups, sweep_row.cuh.
 //  * y / z sweeps (strided directions): an item is a group of 32 adjacent
 //    columns x and a segment along the sweep; each thread marches its column
 //    keeping the stencil in registers.  Loads and stores are coalesced
 //    across the warp (32 consecutive values per component).
-// Both are software-pipelined: the face stage of an iteration uses cell
+// The march is software-pipelined: the face stage of an iteration uses cell
 // stages finished in earlier iterations, so the cell stage (reconstruction
 // + half step) and the face stage (Riemann flux) of one iteration are
 // independent instruction streams the scheduler can interleave.
@@ -47,12 +44,6 @@ constexpr int min_blocks() { return sizeof(T) == 4 ? BAMREX_SWEEP_MIN_BLOCKS_F32
 #endif
 constexpr int kMarchUnroll = BAMREX_MARCH_UNROLL;
 static_assert(kSweepThreads == kStageBlockThreads, "staging sized for the sweep block");
-// Unroll factor of the x-sweep chunk loop.
-#ifndef BAMREX_XCHUNK_UNROLL
-#define BAMREX_XCHUNK_UNROLL 1
-#endif
-constexpr int kXChunkUnroll = BAMREX_XCHUNK_UNROLL;
-
 __device__ __forceinline__ int find_box(const SweepBox* boxes, int nboxes, long long item)
 {
     int lo = 0, hi = nboxes - 1;
@@ -108,17 +99,6 @@ __device__ __forceinline__ void copy_state(const T (&s)[NC], T (&d)[NC])
     for (int n = 0; n < NC; ++n) d[n] = s[n];
 }
 
-template <typename T, int NC>
-__device__ __forceinline__ void shfl_carry(const T (&cur)[NC], const T (&prev)[NC], int lane, int shift,
-                                           T (&out)[NC])
-{
-    // lane t receives cur[t-shift], or prev[32+t-shift] for t < shift
-    const bool from_prev = lane >= 32 - shift;
-#pragma unroll
-    for (int n = 0; n < NC; ++n)
-        out[n] = __shfl_sync(0xffffffffu, from_prev ? prev[n] : cur[n], (lane + 32 - shift) & 31);
-}
-
 // The running maximum of the wave speed |u| + c of a thread's updated cells,
 // in the kernel's own type, without a branch: the value by one comparison,
 // and the largest exponent field beside it (NaN and infinity show there; the
@@ -155,117 +135,6 @@ __device__ __forceinline__ void reduce_ws(const WsMax<T>& w, unsigned long long*
         if (any_bad) atomicMax(dst, 0x7ff8000000000000ull);
         else if (ws > 0.0) atomicMax(dst, (unsigned long long)__double_as_longlong(ws));
     }
-}
-
-// ------------------------------------------------------------------ x sweep
-// Chunk x0, lane t: load A = U(x0+t+2); cell stage of cell x0+t+1; face
-// x0-31+t from the previous chunk's cell stages; update of cell x0-32+t.
-template <typename T, int D, int METHOD, int LIM>
-__global__ void __launch_bounds__(kSweepThreads, min_blocks<T>()) sweep_x_kernel(const SweepArgs a)
-{
-    using S = Scheme<T, D, 0, METHOD, LIM>;
-    constexpr int NC = D + 2;
-    constexpr int H = S::kHalo;
-    StepFactors<T> f;
-    if (!step_factors(a, f)) return;
-    const K<T> k(a.k);
-    const int lane = threadIdx.x & 31;
-    const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    WsMax<T> wsmax;
-
-    for (long long it = gw; it < a.total_items; it += nw) {
-        const int b = a.boxes ? find_box(a.boxes, a.nboxes, it) : 0;
-        const SweepBox& B = a.boxes ? a.boxes[b] : a.one;
-        const long long local = it - B.item_begin;
-        const int seg = (int)(local % B.nseg);
-        const long long row = local / B.nseg;
-        const int ny = B.hi[1] - B.lo[1] + 1;
-        const int j = B.lo[1] + (int)(row % ny);
-        const int kk = B.lo[2] + (int)(row / ny);
-        const int s0 = B.lo[0] + seg * B.seglen;
-        const int s1 = min(s0 + B.seglen, B.hi[0] + 1);
-        const bool last_seg = (s1 == B.hi[0] + 1);
-
-        // row pointers indexed by the absolute x, and the component strides,
-        // held in registers for the whole item
-        const T* __restrict__ in = B.in.ptr<T>() + (long long)(j - B.in.b1) * B.in.js + (long long)(kk - B.in.b2) * B.in.ks - B.in.b0;
-        T* __restrict__ out = B.out.ptr<T>() + (long long)(j - B.out.b1) * B.out.js + (long long)(kk - B.out.b2) * B.out.ks - B.out.b0;
-        T* __restrict__ fl = B.flux.p ? B.flux.ptr<T>() + (long long)(j - B.flux.b1) * B.flux.js + (long long)(kk - B.flux.b2) * B.flux.ks - B.flux.b0 : nullptr;
-        const long long ins = B.in.ns, ons = B.out.ns, fns = B.flux.ns;
-        const bool do_update = a.do_update != 0;
-        const bool ws_on = a.ws_max != nullptr;
-
-        auto load = [&](int x0, T (&u)[NC]) {
-            const int xl = x0 + lane + 2;
-            if (xl >= s0 - H && xl <= s1 - 1 + H) ld_state(in + xl, ins, u);
-            else benign(u);
-        };
-
-        // carried across chunks
-        T Ap[NC];               // previous chunk's loads
-        T ULp[NC], URp[NC];     // previous chunk's cell stages
-        T URpp[NC];             // the chunk before that (its lane 31 is used)
-        T Fp[NC];               // previous chunk's faces (lane 31 used)
-        T Um2p[NC];             // previous chunk's U(x0-32+t)
-        benign(Ap);
-        benign(ULp);
-        benign(URp);
-        benign(URpp);
-        benign(Um2p);
-#pragma unroll
-        for (int n = 0; n < NC; ++n) Fp[n] = T(0);
-
-        T An[NC];
-        load(s0 - 32, An);
-#pragma unroll kXChunkUnroll
-        for (int x0 = s0 - 32; x0 < s1 + 32; x0 += 32) {
-            T A[NC];
-            copy_state(An, A);
-            load(x0 + 32, An);
-            // cell stage of cell x0+t+1 (this chunk)
-            T Um1[NC], Um2[NC];
-            shfl_carry(A, Ap, lane, 1, Um1);  // U(x0+t+1)
-            shfl_carry(A, Ap, lane, 2, Um2);  // U(x0+t)
-            T UL[NC], UR[NC];
-            S::cell(Um2, Um1, A, k, f.hdtdx, UL, UR);
-            // face x0-31+t from the previous chunk: UR(x0-32+t), UL(x0-31+t)
-            T URf[NC];
-            shfl_carry(URp, URpp, lane, 1, URf);
-            T F[NC];
-            S::face(URf, ULp, k, f.half_dx_dt, f.dt_2dx, F);
-            // update of cell o = x0-32+t from faces o and o+1
-            T Fm[NC];
-            shfl_carry(F, Fp, lane, 1, Fm);
-            const int o = x0 - 32 + lane;
-            // the update is computed by every lane (idle lanes hold benign
-            // states) and stored by the lanes that own a cell, so the chunk
-            // stays one basic block
-            const bool upd = do_update && o >= s0 && o < s1;
-            T Un[NC];
-#pragma unroll
-            for (int n = 0; n < NC; ++n) Un[n] = Um2p[n] - f.dtdx * (F[n] - Fm[n]);
-            if (upd) {
-#pragma unroll
-                for (int n = 0; n < NC; ++n) out[o + n * ons] = Un[n];
-            }
-            if (ws_on) wsmax.add(S::speed(Un, k), upd);
-            if (fl) {
-                const int fo = o + 1;
-                if (fo >= s0 && (fo < s1 || (fo == s1 && last_seg))) {
-#pragma unroll
-                    for (int n = 0; n < NC; ++n) fl[fo + n * fns] = F[n];
-                }
-            }
-            copy_state(A, Ap);
-            copy_state(URp, URpp);
-            copy_state(UR, URp);
-            copy_state(UL, ULp);
-            copy_state(F, Fp);
-            copy_state(Um2, Um2p);
-        }
-    }
-    if (a.ws_max) reduce_ws(wsmax, a.ws_max);
 }
 
 // ----------------------------------------------------- marching sweeps

@@ -16,18 +16,18 @@
 namespace bamrex {
 
 template <typename T>
-const void* pick_sweep_kernel(int D, int dir, int method, int fast_lim, bool march);
-extern template const void* pick_sweep_kernel<double>(int, int, int, int, bool);
-extern template const void* pick_sweep_kernel<float>(int, int, int, int, bool);
+const void* pick_sweep_kernel(int D, int dir, int method, int fast_lim, bool march, int rows);
+extern template const void* pick_sweep_kernel<double>(int, int, int, int, bool, int);
+extern template const void* pick_sweep_kernel<float>(int, int, int, int, bool, int);
 
 constexpr int kLaunchThreads = 128;  // kSweepThreads of sweep.cuh
 
 namespace {
 
-const void* pick(int D, int dir, int method, bool fp32, int fast_lim, bool march)
+const void* pick(int D, int dir, int method, bool fp32, int fast_lim, bool march, int rows)
 {
-    return fp32 ? pick_sweep_kernel<float>(D, dir, method, fast_lim, march)
-                : pick_sweep_kernel<double>(D, dir, method, fast_lim, march);
+    return fp32 ? pick_sweep_kernel<float>(D, dir, method, fast_lim, march, rows)
+                : pick_sweep_kernel<double>(D, dir, method, fast_lim, march, rows);
 }
 
 // Resident blocks per SM of each kernel on the current device (with its
@@ -69,7 +69,7 @@ bool tma_requestable(int D, int method, const Consts& k)
 cudaError_t launch_sweep(int D, int dir, int method, bool fp32, const SweepArgs& a, cudaStream_t s, bool march)
 {
     march = march && dir == 0 && D >= 2;
-    const void* fn = pick(D, dir, method, fp32, fast_limiter(D, method, a.k), march);
+    const void* fn = pick(D, dir, method, fp32, fast_limiter(D, method, a.k), march, a.rows);
     if (!fn) return cudaErrorInvalidValue;
     if (a.total_items <= 0) return cudaSuccess;
     const int smem = march ? march_x_smem_bytes(D, fp32) : 0;
@@ -85,7 +85,7 @@ cudaError_t launch_sweep(int D, int dir, int method, bool fp32, const SweepArgs&
 long long sweep_resident_warps(int D, int dir, int method, bool fp32, const Consts& k, bool march)
 {
     march = march && dir == 0 && D >= 2;
-    const void* fn = pick(D, dir, method, fp32, fast_limiter(D, method, k), march);
+    const void* fn = pick(D, dir, method, fp32, fast_limiter(D, method, k), march, kRowsLevel);
     if (!fn) return 0;
     return (long long)device_sm_count() * blocks_per_sm(fn, march ? march_x_smem_bytes(D, fp32) : 0) *
            (kLaunchThreads / 32);

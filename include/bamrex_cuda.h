@@ -198,7 +198,7 @@ typedef struct bamrex_level_desc {
     int method;             /* BAMREX_MUSCL_HANCOCK ... (adv.num_method) */
     double cfl;             /* adv.cfl */
     bamrex_parm parm;
-    int x_segment;          /* cells per warp item in x; 0 = automatic */
+    int x_segment;          /* cells per warp item in x (not ROWS); 0 = automatic */
     int s_segment;          /* cells per thread item in y/z; 0 = automatic */
     int precision;          /* BAMREX_FP64 (0) or BAMREX_FP32_STORAGE */
     int x_mode;             /* BAMREX_XSWEEP_*: kernel of the x sweep; 0 = automatic */
@@ -227,12 +227,11 @@ enum {
     BAMREX_STAGING_WAVE = 3
 };
 
-/* Kernel of a level's x sweep.  ROWS: a warp marches along a row segment,
- * lanes on consecutive cells (best for wide boxes: it spends two extra
- * 32-cell chunks per row segment).  MARCH: each thread marches one row,
- * lanes on 32 adjacent rows (best for levels of narrow boxes, such as
- * max_grid_size 32-128).  AUTO picks by an estimate of the lane slots each
- * spends on the level's boxes.  Both evaluate the same scheme per cell
+/* Register kernel of a level's x sweep.  ROWS: row groups, each lane of a
+ * warp on four consecutive cells of a row (two outside the fast path),
+ * consecutive rows filling the warp.  MARCH: each thread marches one row,
+ * lanes on 32 adjacent rows.  AUTO takes MARCH for levels whose rows are
+ * 24 cells or shorter on average.  Both evaluate the same scheme per cell
  * (results agree to rounding: multiply-add contraction may differ). */
 enum {
     BAMREX_XSWEEP_AUTO = 0,
