@@ -84,6 +84,8 @@ int make_consts(const bamrex_parm* p, int D, Consts& k)
     const double kr = std::nearbyint(k.inv_z);
     if (kr >= 2 && kr <= 16 && std::fabs(k.inv_z - kr) <= 1e-12 * kr) {
         k.root_k = (int)kr;
+        k.root_ik = 1.0 / kr;
+        k.root_c2 = (kr + 1) / (2 * kr * kr);
         k.root_dpos = k.inv_z - kr;
         k.root_dneg = (double)(1.0L / (long double)kr - (long double)k.z);
         k.root_dneg_l2 = (double)((1.0L / (long double)kr - (long double)k.z) * 0.69314718055994530942L);
@@ -219,9 +221,8 @@ int choose_seglen(int dir, const std::vector<bamrex_box>& boxes, long long resid
 // positions, and its halo lanes read the neighbours' rows.  3D 256^3, x sweep
 // by row groups / marching: FP64 in 64^3 boxes 566 / 650 us, 32^3 571 / 673,
 // 16^3 615 / 644, 8^3 894 / 850; FP32 32^3 300 / 433, 16^3 435 / 516, 240^3 in
-// 12^3 701 / 527.  The general path, whose face calls the power functions,
-// gains nothing from four cells per lane: rows up to 512 cells march.
-bool narrow_rows(const std::vector<bamrex_box>& boxes, bool fast)
+// 12^3 701 / 527; general path (gamma 5/3) 1024^2 FP64 in 64^2 boxes 52 / 53.
+bool narrow_rows(const std::vector<bamrex_box>& boxes)
 {
     long long cells = 0, rows = 0;
     for (const auto& b : boxes) {
@@ -229,7 +230,7 @@ bool narrow_rows(const std::vector<bamrex_box>& boxes, bool fast)
         rows += r;
         cells += r * (b.hi[0] - b.lo[0] + 1);
     }
-    return cells <= (fast ? 24 : 512) * rows;
+    return cells <= 24 * rows;
 }
 
 // ---- TMA-staged sweeps (sweep_tma.cuh, sweep_wave.cuh): lane groups and
@@ -1082,7 +1083,7 @@ extern "C" int bamrex_level_create(bamrex_level** out, const bamrex_level_desc* 
     };
     std::vector<SweepBox> sweep_host[3];
     // the register kernel of the x sweep when the caller leaves it open
-    L->x_march = D >= 2 && (desc->x_mode == BAMREX_XSWEEP_MARCH || (desc->x_mode == BAMREX_XSWEEP_AUTO && narrow_rows(L->boxes, fast_limiter(D, L->method, L->k) >= 0)));
+    L->x_march = D >= 2 && (desc->x_mode == BAMREX_XSWEEP_MARCH || (desc->x_mode == BAMREX_XSWEEP_AUTO && narrow_rows(L->boxes)));
     const int row_p = row_positions(fast_limiter(D, L->method, L->k));
     for (int d = 0; d < D; ++d) {
         if (L->sweep_kind[d] >= 0) continue;

@@ -39,6 +39,8 @@ struct Consts {
     double root_dpos;
     double root_dneg_l2;   // root_dneg * ln 2 (applied to log2 x)
     double root_dpos_l2;   // root_dpos * ln 2
+    double root_ik;        // 1 / root_k and (root_k + 1) / (2 root_k^2): the series of
+    double root_c2;        // (1 - e)^(-1/root_k)
     double half_eps;       // 0.5 * epsilon
     double neg_gm1_heps;   // -(gamma - 1) * half_eps
     double one_m_gp1_2g;   // 1 - gp1_2g

@@ -28,7 +28,7 @@ template <typename T>
 struct K {
     T gamma, eps, inv_eps, gm1, half_gm1, z, neg_z, inv_z, gp1_2g, gamma_inv_eps, half_eps;
     T neg_gm1_heps, one_m_gp1_2g;  // -(gamma - 1) eps / 2 and 1 - (gamma + 1) / (2 gamma): the fast path
-    double root_dneg_l2, root_dpos_l2;
+    double root_dneg_l2, root_dpos_l2, root_ik, root_c2;
     int root_k, limiter, uniform_var, need_prim;
     int lim_var[kMaxComp], lim_prim[kMaxComp];
 
@@ -36,7 +36,7 @@ struct K {
         : gamma((T)c.gamma), eps((T)c.eps), inv_eps((T)c.inv_eps), gm1((T)c.gm1), half_gm1((T)c.half_gm1),
           z((T)c.z), neg_z((T)c.neg_z), inv_z((T)c.inv_z), gp1_2g((T)c.gp1_2g), gamma_inv_eps((T)c.gamma_inv_eps),
           half_eps((T)c.half_eps), neg_gm1_heps((T)c.neg_gm1_heps), one_m_gp1_2g((T)c.one_m_gp1_2g),
-          root_dneg_l2(c.root_dneg_l2), root_dpos_l2(c.root_dpos_l2), root_k(c.root_k),
+          root_dneg_l2(c.root_dneg_l2), root_dpos_l2(c.root_dpos_l2), root_ik(c.root_ik), root_c2(c.root_c2), root_k(c.root_k),
           limiter(c.limiter), uniform_var(c.uniform_var), need_prim(c.need_prim)
     {
 #pragma unroll
@@ -56,6 +56,9 @@ __device__ __forceinline__ T sel(const T (&a)[N], int idx)
     for (int m = 1; m < N; ++m) r = (idx == m) ? a[m] : r;
     return r;
 }
+
+template <int D, int DIR>
+struct Prim;
 
 // primv_from_consv (Source/System/Euler/Euler.H:167-198); inv_rho = 1/rho.
 template <typename T, int D>
@@ -86,9 +89,17 @@ __device__ __forceinline__ void phys_flux(const T (&U)[D + 2], const T (&q)[D + 
 template <typename T, int D, int DIR>
 __device__ __forceinline__ void phys_flux(const T (&U)[D + 2], const K<T>& k, T (&F)[D + 2])
 {
-    T q[D + 2], ir;
-    to_prim<T, D>(U, k, q, ir);
-    phys_flux<T, D, DIR>(U, q, k, F);
+    if constexpr (sizeof(T) == 8) {
+        const Prim<D, DIR> q(U, k);
+        F[0] = U[1 + DIR];
+#pragma unroll
+        for (int d = 0; d < D; ++d) F[1 + d] = d == DIR ? fma(q.p, k.inv_eps, q.mnu) : U[1 + DIR] * q.u[d];
+        F[1 + D] = (U[1 + D] + q.p) * q.u[DIR];
+    } else {
+        T q[D + 2], ir;
+        to_prim<T, D>(U, k, q, ir);
+        phys_flux<T, D, DIR>(U, q, k, F);
+    }
 }
 
 // slope_limit<L> (Source/Fluxes/Limiters.H:29-73).
@@ -117,62 +128,8 @@ __device__ __forceinline__ T limiter_value(int lim, T numerator, T denom)
     return slope_limit<T>(lim, numerator / denom);
 }
 
-// ---- gamma powers of the general path ------------------------------------
-template <typename T>
-__device__ __forceinline__ T ipow_k(T y, int k)
-{
-    if (k == 7) {
-        const T y2 = y * y, y3 = y2 * y, y6 = y3 * y3;
-        return y6 * y;
-    }
-    if (k == 5) {
-        const T y2 = y * y, y4 = y2 * y2;
-        return y4 * y;
-    }
-    T r = y;
-    for (int i = 1; i < k; ++i) r *= y;
-    return r;
-}
-
-// x^(-z) for the clamped pressure x >= 1e-14 (HLLC.H:272).  With 1/z ~ k
-// (and T = double), x^(-1/k) comes from a float seed and two Newton steps of
-// y <- y + y (1 - x y^k) / k, then x^(1/k - z) ~ 1 + (1/k - z) ln x.
-template <typename T>
-__device__ __forceinline__ T pow_neg_z(T x, const K<T>& c)
-{
-    if constexpr (sizeof(T) == 4) {
-        return pow(x, c.neg_z);
-    } else {
-        if (c.root_k == 0 || !(x > 1e-30 && x < 1e30)) return pow(x, c.neg_z);
-        const int k = c.root_k;
-        const float lf = __log2f((float)x);
-        double y = (double)exp2f(-lf / (float)k);
-        const double ik = 1.0 / (double)k;
-#pragma unroll
-        for (int it = 0; it < 2; ++it) {
-            const double e = fma(-x, ipow_k(y, k), 1.0);
-            y = fma(y * e, ik, y);
-        }
-        return fma(y, c.root_dneg_l2 * (double)lf, y);
-    }
-}
-
-// b^(1/z) (HLLC.H:270-273): b^k (1 + (1/z - k) ln b) for T = double with an
-// integer k; non-positive or extreme b goes to pow() (a negative base gives
-// NaN there, as in the reference, which then selects q_K = 1).
-template <typename T>
-__device__ __forceinline__ T pow_inv_z(T b, const K<T>& c)
-{
-    if constexpr (sizeof(T) == 4) {
-        return pow(b, c.inv_z);
-    } else {
-        if (c.root_k == 0 || !(b > 1e-30 && b < 1e30)) return pow(b, c.inv_z);
-        const double bk = ipow_k(b, c.root_k);
-        return fma(bk, c.root_dpos_l2 * (double)__log2f((float)b), bk);
-    }
-}
-
 // ---- cell stage: reconstruct_and_half_time_step<limiter,dir> --------------
+// (general path of FP32 storage; FP64: muscl_cell_gen, hllc_face_f64<GEN>)
 // (Source/Fluxes/Flux_Helpers.cpp:92-148) for one cell from its two
 // neighbours along the sweep: returns the half-stepped L/R states.
 template <typename T, int D, int DIR>
@@ -242,8 +199,8 @@ __device__ __forceinline__ void hllc_face(const T (&L)[D + 2], const T (&R)[D + 
     const T icR = (qR[0] >= T(kMinRho)) ? irR : T(1.0 / kMinRho);
     const T cL = sqrt(k.gamma_inv_eps * pL * icL);
     const T cR = sqrt(k.gamma_inv_eps * pR * icR);
-    const T base = (cL + cR - k.half_gm1 * (uR - uL)) / (cL * pow_neg_z<T>(pL, k) + cR * pow_neg_z<T>(pR, k));
-    const T p_rr = pow_inv_z<T>(base, k);
+    const T base = (cL + cR - k.half_gm1 * (uR - uL)) / (cL * pow(pL, k.neg_z) + cR * pow(pR, k.neg_z));
+    const T p_rr = pow(base, k.inv_z);
     const T qwL = (p_rr > pL) ? sqrt(T(1) + k.gp1_2g * (p_rr / pL - T(1))) : T(1);
     const T qwR = (p_rr > pR) ? sqrt(T(1) + k.gp1_2g * (p_rr / pR - T(1))) : T(1);
     const T SL = uL - cL * qwL;
@@ -496,6 +453,28 @@ __device__ __forceinline__ double quarter_limiter(double num, double den, double
     return both_zero(num, den) ? 0.25 : phi;
 }
 
+// The half step of both reconstructed states by the difference of their
+// physical fluxes (Flux_Helpers.cpp:123-148).
+template <int D, int DIR>
+__device__ __forceinline__ void half_step(double (&UL)[D + 2], double (&UR)[D + 2], const K<double>& k, double hdtdx)
+{
+    constexpr int NC = D + 2;
+    constexpr int E = D + 1;
+    const Prim<D, DIR> a(UL, k), b(UR, k);
+    double dF[NC];
+    dF[0] = UR[1 + DIR] - UL[1 + DIR];
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+        dF[1 + d] = d == DIR ? fma(b.p - a.p, k.inv_eps, b.mnu - a.mnu)
+                             : fma(UR[1 + DIR], b.u[d], -(UL[1 + DIR] * a.u[d]));
+    dF[E] = fma(UR[E] + b.p, b.u[DIR], -((UL[E] + a.p) * a.u[DIR]));
+#pragma unroll
+    for (int n = 0; n < NC; ++n) {
+        UL[n] = fma(-hdtdx, dF[n], UL[n]);
+        UR[n] = fma(-hdtdx, dF[n], UR[n]);
+    }
+}
+
 template <int D, int DIR, int LIM>
 __device__ __forceinline__ void muscl_cell_f64(const double (&Um)[D + 2], const double (&U0)[D + 2], const double (&Up)[D + 2],
                                                 const K<double>& k, double hdtdx, double (&UL)[D + 2], double (&UR)[D + 2])
@@ -513,20 +492,112 @@ __device__ __forceinline__ void muscl_cell_f64(const double (&Um)[D + 2], const 
         UL[n] = fma(-qphi, d2[n], U0[n]);
         UR[n] = fma(qphi, d2[n], U0[n]);
     }
-    // the half step by the difference of the two physical fluxes
-    const Prim<D, DIR> a(UL, k), b(UR, k);
-    double dF[NC];
-    dF[0] = UR[1 + DIR] - UL[1 + DIR];
+    half_step<D, DIR>(UL, UR, k, hdtdx);
+}
+
+// quarter_limiter for a limiter known at run time: the same quotients, the
+// operands selected (the limiter is uniform over the launch).
+__device__ __forceinline__ double quarter_limiter_rt(int lim, double num, double den, double sum)
+{
+    const double an = fabs(num), ad = fabs(den);
+    const bool big = an > ad, leer = lim == LIM_VAN_LEER, albada = lim == LIM_VAN_ALBADA, bee = lim == LIM_SUPERBEE;
+    const double top = big ? den : (albada ? num * sum : num);
+    const double bottom = (big || leer) ? sum : (albada ? fma(num, num, den * den) : den);
+    double phi = top * rcp_fast(bottom) * ((big || leer || bee) ? 0.5 : 0.25);
+    phi = (bee && !big && 2.0 * an > ad) ? 0.25 : phi;
+    phi = same_sign(num, den) ? phi : 0.0;
+    return both_zero(num, den) ? 0.25 : phi;
+}
+
+// Cell stage of the general path (any limiting variables, muscl_cell above):
+// one quotient per limiter value and the half step of the fast path.
+template <int D, int DIR>
+__device__ __forceinline__ void muscl_cell_gen(const double (&Um)[D + 2], const double (&U0)[D + 2],
+                                               const double (&Up)[D + 2], const K<double>& k, double hdtdx,
+                                               double (&UL)[D + 2], double (&UR)[D + 2])
+{
+    constexpr int NC = D + 2;
+    double qphi[NC];
+    if (k.uniform_var >= 0) {
+        const int v = k.uniform_var;
+        const double m = sel(Um, v), c = sel(U0, v), p = sel(Up, v);
+        const double q = quarter_limiter_rt(k.limiter, c - m, p - c, p - m);
 #pragma unroll
-    for (int d = 0; d < D; ++d)
-        dF[1 + d] = d == DIR ? fma(b.p - a.p, k.inv_eps, b.mnu - a.mnu)
-                             : fma(UR[1 + DIR], b.u[d], -(UL[1 + DIR] * a.u[d]));
-    dF[E] = fma(UR[E] + b.p, b.u[DIR], -((UL[E] + a.p) * a.u[DIR]));
+        for (int n = 0; n < NC; ++n) qphi[n] = q;
+    } else if (!k.need_prim) {
+#pragma unroll
+        for (int n = 0; n < NC; ++n) {
+            const int v = k.lim_var[n];
+            const double m = v == n ? Um[n] : sel(Um, v), c = v == n ? U0[n] : sel(U0, v), p = v == n ? Up[n] : sel(Up, v);
+            qphi[n] = quarter_limiter_rt(k.limiter, c - m, p - c, p - m);
+        }
+    } else {
+        double Qm[NC], Q0[NC], Qp[NC];
+        auto prim = [&](const double (&U)[NC], double (&q)[NC]) {
+            const Prim<D, DIR> w(U, k);
+            q[0] = U[0];
+#pragma unroll
+            for (int d = 0; d < D; ++d) q[1 + d] = w.u[d];
+            q[1 + D] = w.p;
+        };
+        prim(Um, Qm);
+        prim(U0, Q0);
+        prim(Up, Qp);
+#pragma unroll
+        for (int n = 0; n < NC; ++n) {
+            const int v = k.lim_var[n];
+            const bool pr = k.lim_prim[n] != 0;
+            const double m = pr ? sel(Qm, v) : sel(Um, v), c = pr ? sel(Q0, v) : sel(U0, v), p = pr ? sel(Qp, v) : sel(Up, v);
+            qphi[n] = quarter_limiter_rt(k.limiter, c - m, p - c, p - m);
+        }
+    }
 #pragma unroll
     for (int n = 0; n < NC; ++n) {
-        UL[n] = fma(-hdtdx, dF[n], UL[n]);
-        UR[n] = fma(-hdtdx, dF[n], UR[n]);
+        const double d2 = Up[n] - Um[n];
+        UL[n] = fma(-qphi[n], d2, U0[n]);
+        UR[n] = fma(qphi[n], d2, U0[n]);
     }
+    half_step<D, DIR>(UL, UR, k, hdtdx);
+}
+
+// The powers of the Toro estimate for any gamma: t = w^(-z), 1/w, and
+// b^(1/z) (0 for b <= 0).  With 1/z = root_k to within 1e-12 (gamma = 7/5,
+// 5/3, ...) the iteration of root7 for that k, and to first order the factors
+// w^(1/k - z) = 1 + (1/k - z) ln w and b^(1/z - k) = 1 + (1/z - k) ln b;
+// otherwise, or for extreme arguments, pow().
+__device__ __forceinline__ double ipow(double y, int k)
+{
+    const double y2 = y * y, y4 = y2 * y2;
+    if (k == 7) return y4 * y2 * y;
+    if (k == 5) return y4 * y;
+    double r = y;
+    for (int i = 1; i < k; ++i) r *= y;
+    return r;
+}
+__device__ __forceinline__ void root_gen(double w, const K<double>& c, double& t, double& inv_w)
+{
+    if (c.root_k == 0 || !(w > 1e-30 && w < 1e30)) {
+        t = pow(w, c.neg_z);
+        inv_w = 1.0 / w;
+        return;
+    }
+    const float l2 = log2_hi(w);
+    const float q = -l2 * (float)c.root_ik;
+    const float qr = q + 12582912.0f;
+    const int n = __float_as_int(qr);
+    const int f = __float_as_int(ex2_fast(q - (qr - 12582912.0f)));
+    const double y0 = __hiloint2double((f >> 3) + ((1023 - 127) << 20) + ((n - 0x4b400000) << 20), f << 29);
+    const double yk = ipow(y0, c.root_k);
+    const double e = fma(-w, yk, 1.0);
+    t = fma(y0, fma(e, fma(e, c.root_c2, c.root_ik), c.root_dneg_l2 * (double)l2), y0);
+    inv_w = fma(yk, fma(e, e, e), yk);
+}
+__device__ __forceinline__ double pow_ratio_gen(double b, const K<double>& c)
+{
+    if (!(b > 0.0)) return 0.0;
+    if (c.root_k == 0 || !(b > 1e-30 && b < 1e30)) return pow(b, c.inv_z);
+    const double bk = ipow(b, c.root_k);
+    return fma(bk, c.root_dpos_l2 * (double)log2_hi(b), bk);
 }
 
 // HLLC (hllc_face above, HLLC.cpp:90-172 with HLLC.H:214-337), rearranged to
@@ -542,7 +613,8 @@ __device__ __forceinline__ void muscl_cell_f64(const double (&Um)[D + 2], const 
 //    p* = p_K + eps rho_K (S_K - u_K)(S* - u_K), E* from the energy jump, F =
 //    S* (rho*, rho* u*, E* + p*) + p*/eps; with u_K in place of S* the same
 //    expressions give rho_K, p_K and E_K, so they are the supersonic flux.
-template <int D, int DIR>
+// GEN: any gamma, by root_gen / pow_ratio_gen.
+template <int D, int DIR, bool GEN>
 __device__ __forceinline__ void hllc_face_f64(const double (&L)[D + 2], const double (&R)[D + 2], const K<double>& k,
                                                double (&F)[D + 2])
 {
@@ -558,8 +630,10 @@ __device__ __forceinline__ void hllc_face_f64(const double (&L)[D + 2], const do
     const double cL = sqrt_pos(k.gamma_inv_eps * pL * icL);
     const double cR = sqrt_pos(k.gamma_inv_eps * pR * icR);
     double t, p_lr;  // (p_L / p_R)^z and p_L / p_R
-    root7(pR * rcp_fast(pL), t, p_lr);
-    const double rrL = pow7(fma(-k.half_gm1, uR - uL, cL + cR) * rcp_fast(fma(cR, t, cL)));
+    if constexpr (GEN) root_gen(pR * rcp_fast(pL), k, t, p_lr);
+    else root7(pR * rcp_fast(pL), t, p_lr);
+    const double b = fma(-k.half_gm1, uR - uL, cL + cR) * rcp_fast(fma(cR, t, cL));
+    const double rrL = GEN ? pow_ratio_gen(b, k) : pow7(b);
     const double rrR = rrL * p_lr;
     // q_K = sqrt(1 + (gamma+1)/(2 gamma) (max(p_rr / p_K, 1) - 1)): the select
     // is on the argument (whose value at 1 is exactly 1), since a select
@@ -785,7 +859,8 @@ struct Scheme {
             if constexpr (sizeof(T) == 8) muscl_cell_f64<D, DIR, L>(Um, U0, Up, k, hdtdx, UL, UR);
             else muscl_cell_f32<D, DIR, L>(Um, U0, Up, k, hdtdx, UL, UR);
         } else if constexpr (kReconstruct) {
-            muscl_cell<T, D, DIR>(Um, U0, Up, k, hdtdx, UL, UR);
+            if constexpr (sizeof(T) == 8) muscl_cell_gen<D, DIR>(Um, U0, Up, k, hdtdx, UL, UR);
+            else muscl_cell<T, D, DIR>(Um, U0, Up, k, hdtdx, UL, UR);
         } else {
 #pragma unroll
             for (int n = 0; n < NC; ++n) UL[n] = UR[n] = U0[n];
@@ -797,10 +872,11 @@ struct Scheme {
                                                 T dt_2dx, T (&F)[NC])
     {
         if constexpr (kFast) {
-            if constexpr (sizeof(T) == 8) hllc_face_f64<D, DIR>(L, R, k, F);
+            if constexpr (sizeof(T) == 8) hllc_face_f64<D, DIR, false>(L, R, k, F);
             else hllc_face_f32<D, DIR>(L, R, k, F);
         } else if constexpr (METHOD == M_MUSCL || METHOD == M_HLLC) {
-            hllc_face<T, D, DIR>(L, R, k, F);
+            if constexpr (sizeof(T) == 8) hllc_face_f64<D, DIR, true>(L, R, k, F);
+            else hllc_face<T, D, DIR>(L, R, k, F);
         } else if constexpr (METHOD == M_SLIC || METHOD == M_FORCE) {
             force_face<T, D, DIR>(L, R, k, half_dx_dt, dt_2dx, F);
         } else {

@@ -370,7 +370,7 @@ __global__ void flux_lr_kernel(int lo0, int lo1, int lo2, int hi0, int hi1, int 
             L[n] = pl[n * cL.ns];
             R[n] = pr[n * cR.ns];
         }
-        if (KIND == M_HLLC) hllc_face<double, D, DIR>(L, R, k, F);
+        if (KIND == M_HLLC) hllc_face_f64<D, DIR, true>(L, R, k, F);
         else force_face<double, D, DIR>(L, R, k, half_dx_dt, dt_2dx, F);
         double* pf = flux.ptr<double>() + fab_index(flux, i, j, kk);
         for (int n = 0; n < NC; ++n) pf[n * flux.ns] = F[n];

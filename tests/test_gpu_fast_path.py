@@ -9,14 +9,14 @@ pytestmark = pytest.mark.gpu
 RTOL = 1e-12
 
 
-def _consv(D, q, eps):
+def _consv(D, q, eps, gamma=1.4):
     u = q.copy()
     u[1:1 + D] *= q[0]
-    u[1 + D] = q[1 + D] / 0.4 + 0.5 * eps * q[0] * (q[1:1 + D] ** 2).sum(0)
+    u[1 + D] = q[1 + D] / (gamma - 1) + 0.5 * eps * q[0] * (q[1:1 + D] ** 2).sum(0)
     return u
 
 
-def _states(regime, D, shape, eps, seed):
+def _states(regime, D, shape, eps, seed, gamma=1.4):
     """Primitive plateaus of three cells (so that limited, unlimited and
     exactly flat differences all occur) with a little noise on half of them."""
     rng = np.random.default_rng(seed)
@@ -38,7 +38,7 @@ def _states(regime, D, shape, eps, seed):
         q[1:1 + D] = 0.0
     if regime != "rest":
         q *= 1.0 + 1e-3 * up(rng.uniform(size=coarse) < 0.5) * rng.standard_normal(q.shape)
-    return _consv(D, q, eps)
+    return _consv(D, q, eps, gamma)
 
 
 @pytest.mark.parametrize("regime", ["subsonic", "supersonic_up", "supersonic_down", "pressure_ratio", "rest"])
@@ -65,6 +65,35 @@ def test_fluxes_by_regime(oracle, D, eps, limiter, regime):
         for n in range(D + 2):
             scale = np.max(np.abs(ref[n]))
             assert np.max(np.abs(got[n] - ref[n])) <= RTOL * (scale if scale > 0 else 1.0), (d, n)
+
+
+@pytest.mark.parametrize("regime", ["subsonic", "supersonic_up", "supersonic_down", "pressure_ratio", "rest"])
+@pytest.mark.parametrize("gamma", [5.0 / 3.0, 1.5, 1.25, 1.3], ids=["k5", "k6", "k10", "pow"])
+@pytest.mark.parametrize("limit", ["energy", "own", "primitive"])
+def test_general_path_by_regime(oracle, limit, gamma, regime):
+    """The general path: integer roots 1/z = 5, 6, 10 and pow(), limited on
+    the energy, on each component's own ratio, and on primitive variables."""
+    import torch
+
+    import bamrex_b200 as bx
+    D, shape = 2, (17, 38)
+    kw = {"energy": {}, "own": dict(limiter_indices=list(range(4)) + [0] * 4, limit_on_primv=[False] * 8),
+          "primitive": dict(limiter_indices=[3, 1, 2, 3] + [0] * 4, limit_on_primv=[True] * 4 + [False] * 4)}[limit]
+    lo, hi, begin = (0, 0, 0), (shape[1] - 1, shape[0] - 1, 0), (-2, -2, 0)
+    dx, dt = [0.01] * D, 1e-5
+    for limiter in range(4):
+        u = _states(regime, D, (1, shape[0] + 4, shape[1] + 4), 1.0, 5 + limiter, gamma)
+        ut = torch.tensor(u, device="cuda")
+        for d in range(D):
+            ref = oracle.compute_flux(D, 0, d, lo, hi, u, begin, dx, dt,
+                                      oracle.Parm(D, adiabatic=gamma, limiter=limiter, **kw))
+            ft = torch.full(ref.shape, float("nan"), dtype=torch.float64, device="cuda")
+            bx.compute_flux(0, d, D, (lo, hi), ft, lo, ut, begin, dx, dt,
+                            bx.Parm(D, adiabatic=gamma, limiter=limiter, **kw))
+            got = ft.cpu().numpy()
+            for n in range(D + 2):
+                scale = np.max(np.abs(ref[n]))
+                assert np.max(np.abs(got[n] - ref[n])) <= RTOL * (scale if scale > 0 else 1.0), (limiter, d, n)
 
 
 def test_gamma_beside_seven_fifths(oracle):
