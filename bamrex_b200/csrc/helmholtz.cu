@@ -25,6 +25,7 @@
 #include <cstdint>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -497,6 +498,8 @@ __global__ void prolong_kernel(const HLev F, const HLev C)
         prolong_cell<D>(F, C, c);
 }
 
+#include "helmholtz_tile.cuh"
+
 // The coarse end of a V-cycle in one block: from level 0 of `lv` (the
 // first level of at most kSmallCells cells) down to the bottom and back,
 // every phase a block-strided loop over the level's cells followed by a
@@ -623,6 +626,8 @@ __global__ void __launch_bounds__(kSmallThreads) vcycle_small_kernel(const HLevs
     }
     small_copy(lv.lev[0].phi, S[0].phi, lv.lev[0].ncell);
 }
+
+#include "helmholtz_small.cuh"
 
 // averageDownCoeffs: cell coefficients by the mean of the children, face
 // coefficients by the mean of the fine faces on each coarse face.
@@ -898,6 +903,7 @@ struct bamrex_helmholtz {
     int D = 2;
     HOp op;
     bool staged_smoother = true;  // 2D fused sweeps with cp.async-staged tiles
+    bool tiled_cycle = true;      // 2D levels above those: half a cycle per launch, in tiles
     bool small_cycle = true;      // levels of <= 1024 cells cycled by one block in shared memory
     int nu1 = 2, nu2 = 2, bottom = 16;
     cudaStream_t stream = nullptr;
@@ -1011,30 +1017,105 @@ int smooth(bamrex_helmholtz* H, int l, int sweeps)
     return BAMREX_OK;
 }
 
-int vcycle(bamrex_helmholtz* H, int l)
+int copy_vec(bamrex_helmholtz* H, double* d, const double* s);
+int vcycle_phases(bamrex_helmholtz* H, int l);
+
+// Whether level l's half cycles run as tiles (helmholtz_tile.cuh): 2D, two
+// sweeps each way, no gradient term, even sides (pairs of cells, and red and
+// black keep apart across a periodic seam), not the bottom, and larger than
+// the levels the one-block coarse cycle takes.
+bool tiled_level(const bamrex_helmholtz* H, int l)
+{
+    const HLev& L = H->lev[l];
+    return H->D == 2 && H->tiled_cycle && H->nu1 == 2 && H->nu2 == 2 && L.c == nullptr && l + 1 < (int)H->lev.size() &&
+           L.n[0] % 2 == 0 && L.n[1] % 2 == 0 && L.ncell > kSmallCells;
+}
+
+// The tile kernels' shared memory is above the default limit: raised once per
+// device.
+int tile_smem_ready(bamrex_helmholtz* H)
+{
+    static std::once_flag once[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaError_t e = cudaSuccess;
+    std::call_once(once[dev & 63], [&] {
+        const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        e = cudaFuncSetAttribute(mg_tile_kernel<true, true>, attr, MgWin<true>::kSmem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(mg_tile_kernel<true, false>, attr, MgWin<true>::kSmem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(mg_tile_kernel<false, true>, attr, MgWin<false>::kSmem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(mg_tile_kernel<false, false>, attr, MgWin<false>::kSmem);
+    });
+    return e == cudaSuccess ? BAMREX_OK : hck(H, e, "V-cycle tile shared memory");
+}
+
+// One V-cycle of level l and below from a zero guess: the right-hand side in
+// `rhs`, the result left where *result points (the level's phi or tmp, or
+// `out` when it is given).
+int vcycle(bamrex_helmholtz* H, int l, const double* rhs, double* out, const double** result)
+{
+    HLev& F = H->lev[l];
+    if (tiled_level(H, l)) {
+        const HLev& C = H->lev[l + 1];
+        const int tiles = ((F.n[0] + kMgTile - 1) / kMgTile) * ((F.n[1] + kMgTile - 1) / kMgTile);
+        double* to = out ? out : F.tmp;
+        H_TRY(tile_smem_ready(H));
+        const bool bnd = H->op.bc_lo[0] != BAMREX_LINOP_PERIODIC || H->op.bc_lo[1] != BAMREX_LINOP_PERIODIC;
+        auto down = bnd ? mg_tile_kernel<true, true> : mg_tile_kernel<true, false>;
+        auto up = bnd ? mg_tile_kernel<false, true> : mg_tile_kernel<false, false>;
+        down<<<tiles, kMgThreads, MgWin<true>::kSmem, H->stream>>>(F, H->op, rhs, nullptr, nullptr, F.phi, C);
+        H_TRY(hck(H, cudaGetLastError(), "V-cycle level, down"));
+        const double* coarse = nullptr;
+        H_TRY(vcycle(H, l + 1, C.rhs, nullptr, &coarse));
+        up<<<tiles, kMgThreads, MgWin<false>::kSmem, H->stream>>>(F, H->op, rhs, F.phi, coarse, to, C);
+        *result = to;
+        return hck(H, cudaGetLastError(), "V-cycle level, up");
+    }
+    if (rhs != F.rhs) {
+        // (the finest level: the coarser ones get phi = 0 with their rhs)
+        H_TRY(copy_vec(H, F.rhs, rhs));
+        H_TRY(hck(H, cudaMemsetAsync(F.phi, 0, sizeof(double) * F.ncell, H->stream), "memset"));
+    }
+    H_TRY(vcycle_phases(H, l));
+    *result = F.phi;
+    if (out) {
+        H_TRY(copy_vec(H, out, F.phi));
+        *result = out;
+    }
+    return BAMREX_OK;
+}
+
+// The same as grid-wide phases on the level's own arrays.
+int vcycle_phases(bamrex_helmholtz* H, int l)
 {
     const int nl = (int)H->lev.size();
     if (H->small_cycle && H->lev[l].ncell <= kSmallCells && nl - l <= kSmallLevels) {
         // the rest of the cycle in one block, its levels in shared memory
         HLevs lv;
         lv.n = nl - l;
+        const bool plain2 = H->D == 2 && H->lev[l].c == nullptr;
         long long doubles = 0;
         for (int q = l; q < nl; ++q) {
             lv.lev[q - l] = H->lev[q];
-            doubles += small_level_doubles(H->lev[q], H->D);
+            doubles += plain2 ? small2_level_doubles(H->lev[q]) : small_level_doubles(H->lev[q], H->D);
         }
         const long long bytes = doubles * (long long)sizeof(double);
         if (bytes <= kSmallSmemMax) {
-            static bool attr_set[2][64] = { { false } };
+            static bool attr_set[4][64] = { { false } };
             int dev = 0;
             cudaGetDevice(&dev);
-            const void* fn = H->D == 3 ? (const void*)vcycle_small_kernel<3> : (const void*)vcycle_small_kernel<2>;
-            if (!attr_set[H->D == 3][dev & 63]) {
-                H_TRY(hck(H, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmemMax),
+            const bool bnd = H->op.bc_lo[0] != BAMREX_LINOP_PERIODIC || H->op.bc_lo[1] != BAMREX_LINOP_PERIODIC;
+            const int kind = plain2 ? (bnd ? 3 : 2) : H->D == 3 ? 1 : 0;
+            const void* fns[4] = { (const void*)vcycle_small_kernel<2>, (const void*)vcycle_small_kernel<3>,
+                                   (const void*)vcycle_small2_kernel<false>, (const void*)vcycle_small2_kernel<true> };
+            if (!attr_set[kind][dev & 63]) {
+                H_TRY(hck(H, cudaFuncSetAttribute(fns[kind], cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmemMax),
                           "coarse V-cycle shared memory"));
-                attr_set[H->D == 3][dev & 63] = true;
+                attr_set[kind][dev & 63] = true;
             }
-            if (H->D == 3)
+            auto small2 = bnd ? vcycle_small2_kernel<true> : vcycle_small2_kernel<false>;
+            if (plain2) small2<<<1, kSmall2Threads, (size_t)bytes, H->stream>>>(lv, H->op, H->nu1, H->nu2, H->bottom);
+            else if (H->D == 3)
                 vcycle_small_kernel<3><<<1, kSmallThreads, (size_t)bytes, H->stream>>>(lv, H->op, H->nu1, H->nu2, H->bottom);
             else
                 vcycle_small_kernel<2><<<1, kSmallThreads, (size_t)bytes, H->stream>>>(lv, H->op, H->nu1, H->nu2, H->bottom);
@@ -1043,14 +1124,16 @@ int vcycle(bamrex_helmholtz* H, int l)
     }
     if (l == nl - 1) return smooth(H, l, H->bottom);
     H_TRY(smooth(H, l, H->nu1));
-    const HLev& F = H->lev[l];
-    const HLev& C = H->lev[l + 1];
+    HLev F = H->lev[l];
+    HLev C = H->lev[l + 1];
     H_TRY(launch_apply(H, l, F.phi, F.res, F.rhs, 1));
     const int g = grid_for(C.ncell);
     if (H->D == 3) restrict_kernel<3><<<g, kThreads, 0, H->stream>>>(F, C);
     else restrict_kernel<2><<<g, kThreads, 0, H->stream>>>(F, C);
     H_TRY(hck(H, cudaGetLastError(), "restrict"));
-    H_TRY(vcycle(H, l + 1));
+    const double* coarse = nullptr;
+    H_TRY(vcycle(H, l + 1, C.rhs, nullptr, &coarse));
+    C.phi = const_cast<double*>(coarse);
     const int gf = grid_for(F.ncell);
     if (H->D == 3) prolong_kernel<3><<<gf, kThreads, 0, H->stream>>>(F, C);
     else prolong_kernel<2><<<gf, kThreads, 0, H->stream>>>(F, C);
@@ -1086,14 +1169,11 @@ int copy_vec(bamrex_helmholtz* H, double* d, const double* s)
     return hck(H, cudaGetLastError(), "copy");
 }
 
-// z = M y: one V-cycle from a zero guess
+// z = M y: one V-cycle from a zero guess (z and y are distinct vectors)
 int precondition(bamrex_helmholtz* H, double* z, const double* y)
 {
-    const HLev& F = H->lev[0];
-    H_TRY(copy_vec(H, F.rhs, y));
-    H_TRY(hck(H, cudaMemsetAsync(F.phi, 0, sizeof(double) * F.ncell, H->stream), "memset"));
-    H_TRY(vcycle(H, 0));
-    return copy_vec(H, z, F.phi);
+    const double* r = nullptr;
+    return vcycle(H, 0, y, z, &r);
 }
 
 // One BiCGStab iteration (right preconditioning), all scalars on the device.
