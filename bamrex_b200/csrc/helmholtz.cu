@@ -106,38 +106,71 @@ __device__ __forceinline__ ApplyCoef apply_coef(const HLev& L, const HOp& op)
     return a;
 }
 
-// (A x)_c, or rhs_c - (A x)_c with mode 1.
+// The position of cell c, by 32-bit divisions where the level allows.
 template <int D>
+__device__ __forceinline__ void cell_at(const HLev& L, long long c, int& i, int& j, int& k)
+{
+    if (L.ncell >> 31) {
+        i = (int)(c % L.n[0]);
+        j = (int)((c / L.n[0]) % L.n[1]);
+        k = (int)(c / ((long long)L.n[0] * L.n[1]));
+        return;
+    }
+    const unsigned u = (unsigned)c, row = u / (unsigned)L.n[0];
+    i = (int)(u - row * (unsigned)L.n[0]);
+    k = D > 2 ? (int)(row / (unsigned)L.n[1]) : 0;
+    j = (int)row - k * L.n[1];
+}
+
+// (A x)_c, or rhs_c - (A x)_c with mode 1.  GLOBAL: the vectors and
+// coefficients lie in global memory and are not written by the launch (loads
+// by the read-only path, which a loop over cells may issue ahead of its
+// stores); otherwise in shared memory.
+template <bool GLOBAL>
+__device__ __forceinline__ double ld_val(const double* p)
+{
+    if constexpr (GLOBAL) return __ldg(p);
+    else return *p;
+}
+
+template <int D, bool GLOBAL = true>
 __device__ __forceinline__ double apply_value(const HLev& L, const HOp& op, const ApplyCoef& ac,
                                               const double* __restrict__ x, const double* __restrict__ rhs, int mode,
                                               long long c)
 {
     const double* dxinv = ac.dxinv;
     const double* dh = ac.dh;
-    {
-        const int i = (int)(c % L.n[0]);
-        const int j = (int)((c / L.n[0]) % L.n[1]);
-        const int k = (int)(c / ((long long)L.n[0] * L.n[1]));
-        const double xc = x[c];
-        double xm[3], xp[3], cf;
-        for (int d = 0; d < D; ++d) {
-            xm[d] = nbr(x, L, op, i, j, k, d, -1, xc, cf);
-            xp[d] = nbr(x, L, op, i, j, k, d, +1, xc, cf);
-        }
-        double v = op.ascal * L.a[c] * xc;
-        for (int d = 0; d < D; ++d) {
-            const int ih = i + (d == 0), jh = j + (d == 1), kh = k + (d == 2);
-            const double bl = L.b[d][fidx(L, d, i, j, k)], bh = L.b[d][fidx(L, d, ih, jh, kh)];
-            v = v - dh[d] * (bh * (xp[d] - xc) - bl * (xc - xm[d]));
-        }
-        if (L.c) {
-            for (int d = 0; d < D; ++d) {
-                const double chd = op.cscal * L.c[(long long)d * L.ncell + c] * 0.5 * dxinv[d];
-                v = v + chd * (xp[d] - xm[d]);
-            }
-        }
-        return mode ? rhs[c] - v : v;
+    const double* __restrict__ a = L.a;
+    int i, j, k;
+    cell_at<D>(L, c, i, j, k);
+    const double xc = ld_val<GLOBAL>(x + c);
+    double xm[3], xp[3], bl[3], bh[3];
+    long long stride = 1;
+    const int pos[3] = { i, j, k };
+    for (int d = 0; d < D; ++d) {
+        auto at = [&](int s) {
+            const int q = pos[d] + s;
+            if (q >= 0 && q < L.n[d]) return ld_val<GLOBAL>(x + c + s * stride);
+            const int bc = s < 0 ? op.bc_lo[d] : op.bc_hi[d];
+            if (bc == BAMREX_LINOP_PERIODIC) return ld_val<GLOBAL>(x + c - s * (L.n[d] - 1) * stride);
+            return (bc == BAMREX_LINOP_NEUMANN ? 1.0 : -1.0) * xc;
+        };
+        xm[d] = at(-1);
+        xp[d] = at(+1);
+        const double* __restrict__ b = L.b[d];
+        bl[d] = ld_val<GLOBAL>(b + fidx(L, d, i, j, k));
+        bh[d] = ld_val<GLOBAL>(b + fidx(L, d, i + (d == 0), j + (d == 1), k + (d == 2)));
+        stride *= L.n[d];
     }
+    double v = op.ascal * ld_val<GLOBAL>(a + c) * xc;
+    for (int d = 0; d < D; ++d) v = v - dh[d] * (bh[d] * (xp[d] - xc) - bl[d] * (xc - xm[d]));
+    if (L.c) {
+        for (int d = 0; d < D; ++d) {
+            const double chd = op.cscal * ld_val<GLOBAL>(L.c + (long long)d * L.ncell + c) * 0.5 * dxinv[d];
+            v = v + chd * (xp[d] - xm[d]);
+        }
+    }
+    return mode ? ld_val<GLOBAL>(rhs + c) - v : v;
 }
 
 template <int D>
@@ -611,7 +644,7 @@ __global__ void __launch_bounds__(kSmallThreads) vcycle_small_kernel(const HLevs
         const HLev C = S[l + 1];
         small_sweeps<D>(F, op, nu1);
         const ApplyCoef ac = apply_coef(F, op);
-        for (int c = threadIdx.x; c < (int)F.ncell; c += blockDim.x) F.res[c] = apply_value<D>(F, op, ac, F.phi, F.rhs, 1, c);
+        for (int c = threadIdx.x; c < (int)F.ncell; c += blockDim.x) F.res[c] = apply_value<D, false>(F, op, ac, F.phi, F.rhs, 1, c);
         __syncthreads();
         for (int c = threadIdx.x; c < (int)C.ncell; c += blockDim.x) restrict_cell<D>(F, C, c);
         __syncthreads();
@@ -716,6 +749,79 @@ struct KScal {
     int pad;
 };
 
+// The block's part of NS dot products, and in the last block to arrive their
+// sums and what `op` does with them: the partials and trees of
+// dot_partial_kernel / dot_final_kernel (the same grid), so the sums are the
+// same bits, without the second launch and with the vectors read where they
+// are made.
+enum { kDotRv, kDotTsTt, kDotRrRho };
+
+template <int NS>
+__device__ __forceinline__ void dot_finish(double (&acc)[NS], double* __restrict__ part, unsigned* counter, KScal* S, int op)
+{
+    __shared__ double red[NS][kThreads];
+    __shared__ bool last;
+    auto tree = [&]() {
+        __syncthreads();
+        for (int w = kThreads / 2; w > 0; w >>= 1) {
+            if (threadIdx.x < w)
+                for (int m = 0; m < NS; ++m) red[m][threadIdx.x] = red[m][threadIdx.x] + red[m][threadIdx.x + w];
+            __syncthreads();
+        }
+    };
+    for (int m = 0; m < NS; ++m) red[m][threadIdx.x] = acc[m];
+    tree();
+    if (threadIdx.x == 0) {
+        for (int m = 0; m < NS; ++m) part[m * gridDim.x + blockIdx.x] = red[m][0];
+        __threadfence();
+        last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int m = 0; m < NS; ++m) {
+        double t = 0.0;
+        for (int q = threadIdx.x; q < (int)gridDim.x; q += kThreads) t = t + __ldcg(part + m * gridDim.x + q);
+        red[m][threadIdx.x] = t;
+    }
+    tree();
+    if (threadIdx.x == 0) {
+        *counter = 0;
+        if (op == kDotRv) {
+            S->rv = red[0][0];
+        } else if (op == kDotTsTt) {
+            S->ts = red[0][0];
+            S->tt = red[NS - 1][0];
+        } else {
+            // after x and r: alpha and omega of this iteration, and the next
+            // one's rho
+            S->rr = red[0][0];
+            S->alpha = S->rho / S->rv;
+            S->omega = S->ts / S->tt;
+            S->rho_old = S->rho;
+            S->rho = red[NS - 1][0];
+        }
+    }
+}
+
+// y = A x with (w, y), and with (y, y) when NS = 2
+template <int D, int NS>
+__global__ void __launch_bounds__(kThreads) apply_dot_kernel(const HLev L, const HOp op, const double* __restrict__ x,
+                                                             double* __restrict__ y, const double* __restrict__ w,
+                                                             double* __restrict__ part, unsigned* counter, KScal* S)
+{
+    const ApplyCoef ac = apply_coef(L, op);
+    double acc[NS] = {};
+#pragma unroll 2
+    for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < L.ncell; c += (long long)gridDim.x * blockDim.x) {
+        const double v = apply_value<D>(L, op, ac, x, nullptr, 0, c);
+        y[c] = v;
+        acc[0] = acc[0] + (NS == 1 ? w[c] * v : v * w[c]);
+        if (NS == 2) acc[NS - 1] = acc[NS - 1] + v * v;
+    }
+    dot_finish<NS>(acc, part, counter, S, NS == 1 ? kDotRv : kDotTsTt);
+}
+
 __global__ void bicg_p_kernel(double* __restrict__ p, const double* __restrict__ r, const double* __restrict__ v,
                               const KScal* __restrict__ S, long long n)
 {
@@ -734,28 +840,25 @@ __global__ void bicg_s_kernel(double* __restrict__ s, const double* __restrict__
         s[c] = r[c] - alpha * v[c];
 }
 
-// x += alpha phat + omega shat; r = s - omega t
-__global__ void bicg_xr_kernel(double* __restrict__ x, double* __restrict__ r, const double* __restrict__ ph,
-                               const double* __restrict__ sh, const double* __restrict__ s,
-                               const double* __restrict__ t, const KScal* __restrict__ S, long long n)
+// x += alpha phat + omega shat; r = s - omega t; (r, r) and (rhat, r)
+__global__ void __launch_bounds__(kThreads) bicg_xr_kernel(double* __restrict__ x, double* __restrict__ r,
+                                                           const double* __restrict__ ph, const double* __restrict__ sh,
+                                                           const double* __restrict__ s, const double* __restrict__ t,
+                                                           const double* __restrict__ rh, KScal* S, long long n,
+                                                           double* __restrict__ part, unsigned* counter)
 {
     const double alpha = S->rho / S->rv;
     const double omega = S->ts / S->tt;
+    double acc[2] = {};
     for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n;
          c += (long long)gridDim.x * blockDim.x) {
         x[c] = x[c] + alpha * ph[c] + omega * sh[c];
-        r[c] = s[c] - omega * t[c];
+        const double v = s[c] - omega * t[c];
+        r[c] = v;
+        acc[0] = acc[0] + v * v;
+        acc[1] = acc[1] + rh[c] * v;
     }
-}
-
-__global__ void bicg_scalars_kernel(KScal* S, int stage)
-{
-    if (stage == 0) {  // start of an iteration after the first
-        S->rho_old = S->rho;
-    } else if (stage == 1) {  // after (t,s) and (t,t): omega for the next iteration
-        S->alpha = S->rho / S->rv;
-        S->omega = S->ts / S->tt;
-    }
+    dot_finish<2>(acc, part, counter, S, kDotRrRho);
 }
 
 __global__ void copy_kernel(double* __restrict__ d, const double* __restrict__ s, long long n)
@@ -915,7 +1018,8 @@ struct bamrex_helmholtz {
     // Krylov vectors on the finest level
     double *x = nullptr, *r = nullptr, *rh = nullptr, *p = nullptr, *v = nullptr, *ph = nullptr, *s = nullptr,
            *sh = nullptr, *t = nullptr, *bvec = nullptr;
-    double* part = nullptr;
+    double* part = nullptr;        // dot-product partials (two sums)
+    unsigned* counter = nullptr;   // blocks arrived in a fused dot product
     KScal* d_scal = nullptr;
     KScal* h_scal = nullptr;  // pinned
     std::vector<double*> cbufs;  // per level, D * ncell: the C coefficients
@@ -1182,25 +1286,25 @@ int bicg_iteration(bamrex_helmholtz* H)
     const long long n = H->lev[0].ncell;
     const int g = grid_for(n);
     KScal* S = H->d_scal;
-    bicg_scalars_kernel<<<1, 1, 0, H->stream>>>(S, 0);
-    H_TRY(hck(H, cudaGetLastError(), "scalars"));
-    H_TRY(dot(H, H->rh, H->r, &S->rho));
+    auto apply_dot = [&](const double* x, double* y, const double* w, bool yy) {
+        const HLev& L = H->lev[0];
+        auto fn = H->D == 3 ? (yy ? apply_dot_kernel<3, 2> : apply_dot_kernel<3, 1>)
+                            : (yy ? apply_dot_kernel<2, 2> : apply_dot_kernel<2, 1>);
+        fn<<<kDotBlocks, kThreads, 0, H->stream>>>(L, H->op, x, y, w, H->part, H->counter, S);
+        return hck(H, cudaGetLastError(), "apply and dot");
+    };
+    // rho = (rhat, r) is there: from the solve's start or the last iteration
     bicg_p_kernel<<<g, kThreads, 0, H->stream>>>(H->p, H->r, H->v, S, n);
     H_TRY(hck(H, cudaGetLastError(), "bicg p"));
     H_TRY(precondition(H, H->ph, H->p));
-    H_TRY(launch_apply(H, 0, H->ph, H->v, nullptr, 0));
-    H_TRY(dot(H, H->rh, H->v, &S->rv));
+    H_TRY(apply_dot(H->ph, H->v, H->rh, false));
     bicg_s_kernel<<<g, kThreads, 0, H->stream>>>(H->s, H->r, H->v, S, n);
     H_TRY(hck(H, cudaGetLastError(), "bicg s"));
     H_TRY(precondition(H, H->sh, H->s));
-    H_TRY(launch_apply(H, 0, H->sh, H->t, nullptr, 0));
-    H_TRY(dot(H, H->t, H->s, &S->ts));
-    H_TRY(dot(H, H->t, H->t, &S->tt));
-    bicg_xr_kernel<<<g, kThreads, 0, H->stream>>>(H->x, H->r, H->ph, H->sh, H->s, H->t, S, n);
-    H_TRY(hck(H, cudaGetLastError(), "bicg xr"));
-    bicg_scalars_kernel<<<1, 1, 0, H->stream>>>(S, 1);
-    H_TRY(hck(H, cudaGetLastError(), "scalars"));
-    return dot(H, H->r, H->r, &S->rr);
+    H_TRY(apply_dot(H->sh, H->t, H->s, true));
+    bicg_xr_kernel<<<kDotBlocks, kThreads, 0, H->stream>>>(H->x, H->r, H->ph, H->sh, H->s, H->t, H->rh, S, n, H->part,
+                                                          H->counter);
+    return hck(H, cudaGetLastError(), "bicg x, r");
 }
 
 bool is_device_ptr(const void* p)
@@ -1297,8 +1401,9 @@ extern "C" int bamrex_helmholtz_create(bamrex_helmholtz** out, const bamrex_helm
     const long long n0 = H->lev[0].ncell;
     size_t ov[10];
     for (int q = 0; q < 10; ++q) ov[q] = take(sizeof(double) * n0);
-    const size_t opart = take(sizeof(double) * kDotBlocks);
+    const size_t opart = take(sizeof(double) * 2 * kDotBlocks);
     const size_t oscal = take(sizeof(KScal));
+    const size_t ocount = take(sizeof(unsigned));
     cudaError_t e = cudaMalloc((void**)&H->arena, off);
     if (e != cudaSuccess) return fail(BAMREX_ERR_OOM, std::string("cudaMalloc of the Helmholtz arena failed: ") + cudaGetErrorString(e));
     e = cudaMallocHost((void**)&H->h_scal, sizeof(KScal));
@@ -1323,6 +1428,7 @@ extern "C" int bamrex_helmholtz_create(bamrex_helmholtz** out, const bamrex_helm
     for (int q = 0; q < 10; ++q) *vv[q] = (double*)(A + ov[q]);
     H->part = (double*)(A + opart);
     H->d_scal = (KScal*)(A + oscal);
+    H->counter = (unsigned*)(A + ocount);
     e = cudaMemset(H->arena, 0, off);
     if (e != cudaSuccess) {
         cudaFree(H->arena);
@@ -1548,11 +1654,12 @@ extern "C" int bamrex_helmholtz_solve(bamrex_helmholtz* H, double* x, const doub
     H_TRY(hck(H, cudaMemsetAsync(H->v, 0, sizeof(double) * n, H->stream), "memset"));
     KScal init;
     std::memset(&init, 0, sizeof(init));
-    init.rho = init.alpha = init.omega = init.rv = init.ts = init.tt = 1.0;
+    init.rho = init.rho_old = init.alpha = init.omega = init.rv = init.ts = init.tt = 1.0;
     *H->h_scal = init;
     H_TRY(hck(H, cudaMemcpyAsync(S, H->h_scal, sizeof(KScal), cudaMemcpyHostToDevice, H->stream), "scalars"));
     H_TRY(dot(H, H->bvec, H->bvec, &S->bb));
     H_TRY(dot(H, H->r, H->r, &S->rr));
+    H_TRY(dot(H, H->rh, H->r, &S->rho));  // rho_old stays 1
     H_TRY(hck(H, cudaMemcpyAsync(H->h_scal, S, sizeof(KScal), cudaMemcpyDeviceToHost, H->stream), "scalars"));
     H_TRY(hck(H, cudaStreamSynchronize(H->stream), "sync"));
     const double bnorm = std::sqrt(H->h_scal->bb);
