@@ -1888,50 +1888,103 @@ extern "C" int bamrex_level_est_time_step(bamrex_level* L, double* dt_est)
     return BAMREX_OK;
 }
 
+// A run as line_run.cu's single block: a 1D level that is one box over its
+// domain, with nothing else to do in a step (no body, no registers, no other
+// rank's ghost cells, no per-sweep timing).  The line is drawn at four passes
+// of the block, 1920 cells: there a step takes 5.5 us (FP64 MUSCL-Hancock) or
+// 11.4 (its general path, the slowest) against 10.3 - 12.3 and 14.4 as three
+// launches; at 2880 cells 7.8 and 16.7 against 10.3 and 13.2.
+static bool line_run(const bamrex_level* L)
+{
+    return L->D == 1 && L->boxes.size() == 1 && L->boxes[0].lo[0] == L->domain.lo[0] &&
+           L->boxes[0].hi[0] == L->domain.hi[0] && line_run_supported((int)L->ncells) && !L->body && !L->timing &&
+           L->reg_tasks[0].empty() && !L->halo_send[0].nops && !L->halo_recv[0].nops && !L->d_split[0][0][0];
+}
+
+static int line_run_enqueue(bamrex_level* L, int nsteps, double stop_time, double start_time)
+{
+    // a launch's steps: a few ms of work; even, so that each starts from the
+    // same buffer
+    constexpr int kSteps = 4096;
+    const bamrex_box& B = L->boxes[0];
+    auto first = [&](const FabDev& f) {
+        return (char*)f.p + ((long long)(B.lo[0] - f.b0) + (B.lo[1] - f.b1) * f.js + (B.lo[2] - f.b2) * f.ks) * (long long)L->esize;
+    };
+    const FabDev &in = L->fab[L->cur][0], &out = L->fab[L->cur ^ 1][0];
+    LineArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.in = first(in);
+    a.out = first(out);
+    a.in_ns = in.ns;
+    a.out_ns = out.ns;
+    a.n = (int)L->ncells;
+    a.init = true;
+    a.time = start_time;
+    a.stop_time = stop_time;
+    a.dx = L->dx[0];
+    a.cfl = L->cfl;
+    a.bc_lo = L->bc_lo[0];
+    a.bc_hi = L->bc_hi[0];
+    a.scal = L->d_scal;
+    a.k = L->k;
+    do {
+        a.nsteps = std::min(nsteps, kSteps);
+        BX_TRY(level_launch(L, launch_line_run(L->method, L->fp32, a, L->stream), "line run"));
+        nsteps -= a.nsteps;
+        a.init = false;
+    } while (nsteps > 0);
+    return BAMREX_OK;
+}
+
 extern "C" int bamrex_level_run_async(bamrex_level* L, int nsteps, double stop_time, int use_graph, double start_time)
 {
     if (!L) return fail(BAMREX_ERR_ARG, "NULL level");
     if (nsteps < 0) return L->set_err(fail(BAMREX_ERR_ARG, "nsteps must be >= 0"));
     if (L->run_pending) return L->set_err(fail(BAMREX_ERR_ARG, "a run is pending: call bamrex_level_run_wait"));
     StepScalars* h = L->h_scal;
-    std::memset(h, 0, sizeof(*h));
-    h->time = start_time;
-    h->stop_time = stop_time;
-    cudaError_t e = cudaMemcpyAsync(L->d_scal, h, sizeof(StepScalars), cudaMemcpyHostToDevice, L->stream);
-    if (e != cudaSuccess) return L->set_err(cuda_fail(e, "scalars upload"));
-    // computeInitialDt from the current state
-    BX_TRY(level_launch(L, launch_max_wave_speed(L->D, L->fp32, fast_limiter(L->D, L->method, L->k) >= 0, L->d_fab[L->cur], L->d_pack, (int)L->boxes.size(), L->ncells, L->k,
-                                                 &L->d_scal->ws_bits, L->d_scal, L->stream),
-                        "max wave speed"));
-    BX_TRY(level_launch(L, launch_step_dt(L->d_scal, L->D, L->dx[0], L->dx[1], L->dx[2], L->cfl, 0, L->stream), "step dt"));
     const int start = L->cur;
-    int p = start;
-    for (int s = 0; s < nsteps; ++s) {
-        if (use_graph) {
-            if (!L->graph[p]) {
-                cudaGraph_t gr = nullptr;
-                e = cudaStreamBeginCapture(L->stream, cudaStreamCaptureModeThreadLocal);
-                if (e != cudaSuccess) return L->set_err(cuda_fail(e, "begin capture"));
-                const long long before = L->launches;
-                const int rc = level_step(L, p, 0.0, L->d_scal, false);
-                e = cudaStreamEndCapture(L->stream, &gr);
-                if (rc != BAMREX_OK) {
-                    if (gr) cudaGraphDestroy(gr);
-                    return rc;
+    cudaError_t e = cudaSuccess;
+    if (line_run(L)) {
+        BX_TRY(line_run_enqueue(L, nsteps, stop_time, start_time));
+    } else {
+        std::memset(h, 0, sizeof(*h));
+        h->time = start_time;
+        h->stop_time = stop_time;
+        e = cudaMemcpyAsync(L->d_scal, h, sizeof(StepScalars), cudaMemcpyHostToDevice, L->stream);
+        if (e != cudaSuccess) return L->set_err(cuda_fail(e, "scalars upload"));
+        // computeInitialDt from the current state
+        BX_TRY(level_launch(L, launch_max_wave_speed(L->D, L->fp32, fast_limiter(L->D, L->method, L->k) >= 0, L->d_fab[L->cur], L->d_pack, (int)L->boxes.size(), L->ncells, L->k,
+                                                     &L->d_scal->ws_bits, L->d_scal, L->stream),
+                            "max wave speed"));
+        BX_TRY(level_launch(L, launch_step_dt(L->d_scal, L->D, L->dx[0], L->dx[1], L->dx[2], L->cfl, 0, L->stream), "step dt"));
+        int p = start;
+        for (int s = 0; s < nsteps; ++s) {
+            if (use_graph) {
+                if (!L->graph[p]) {
+                    cudaGraph_t gr = nullptr;
+                    e = cudaStreamBeginCapture(L->stream, cudaStreamCaptureModeThreadLocal);
+                    if (e != cudaSuccess) return L->set_err(cuda_fail(e, "begin capture"));
+                    const long long before = L->launches;
+                    const int rc = level_step(L, p, 0.0, L->d_scal, false);
+                    e = cudaStreamEndCapture(L->stream, &gr);
+                    if (rc != BAMREX_OK) {
+                        if (gr) cudaGraphDestroy(gr);
+                        return rc;
+                    }
+                    if (e != cudaSuccess) return L->set_err(cuda_fail(e, "end capture"));
+                    L->launches = before;  // counted per replay below
+                    e = cudaGraphInstantiate(&L->graph[p], gr, 0);
+                    cudaGraphDestroy(gr);
+                    if (e != cudaSuccess) return L->set_err(cuda_fail(e, "graph instantiate"));
                 }
-                if (e != cudaSuccess) return L->set_err(cuda_fail(e, "end capture"));
-                L->launches = before;  // counted per replay below
-                e = cudaGraphInstantiate(&L->graph[p], gr, 0);
-                cudaGraphDestroy(gr);
-                if (e != cudaSuccess) return L->set_err(cuda_fail(e, "graph instantiate"));
+                e = cudaGraphLaunch(L->graph[p], L->stream);
+                if (e != cudaSuccess) return L->set_err(cuda_fail(e, "graph launch"));
+                L->launches += 2 * L->D + 1;
+            } else {
+                BX_TRY(level_step(L, p, 0.0, L->d_scal, true));
             }
-            e = cudaGraphLaunch(L->graph[p], L->stream);
-            if (e != cudaSuccess) return L->set_err(cuda_fail(e, "graph launch"));
-            L->launches += 2 * L->D + 1;
-        } else {
-            BX_TRY(level_step(L, p, 0.0, L->d_scal, true));
+            p ^= (L->D & 1);
         }
-        p ^= (L->D & 1);
     }
     e = cudaMemcpyAsync(h, L->d_scal, sizeof(StepScalars), cudaMemcpyDeviceToHost, L->stream);
     if (e != cudaSuccess) return L->set_err(cuda_fail(e, "scalars readback"));

@@ -98,6 +98,35 @@ struct StepScalars {
     int pad;
 };
 
+#ifdef __CUDACC__
+// The next dt from the max wave speed in ws_bits: cfl * min_d dx_d / max_speed,
+// then the stop-time clamp of computeInitialDt / computeNewDt
+// (Source/AmrLevelAdv.cpp:513-523, 600-611); end_step: of the step just done.
+__device__ __forceinline__ void next_step_scalars(StepScalars& s, int D, const double (&dxs)[3], double cfl, bool end_step)
+{
+    if (end_step) {
+        s.time = s.time + s.dt;
+        s.steps += 1;
+    }
+    const double ms = __longlong_as_double((long long)s.ws_bits);
+    double dt_est = 1.0e20;
+    for (int d = 0; d < D; ++d) dt_est = fmin(dt_est, dxs[d] / ms);
+    dt_est *= cfl;
+    double dt_0 = dt_est;
+    if (s.stop_time >= 0.0) {
+        const double eps = 0.001 * dt_0;
+        if ((s.time + dt_0) > (s.stop_time - eps)) dt_0 = s.stop_time - s.time;
+        if (!(s.time < s.stop_time)) s.done = 1;
+    }
+    if (!(dt_est > 0.0) || dt_est != dt_est || isinf(dt_est)) {
+        s.status = 3; /* BAMREX_ERR_NAN */
+        s.done = 1;
+    }
+    s.dt = dt_0;
+    s.ws_bits = 0ull;
+}
+#endif
+
 struct SweepArgs {
     const SweepBox* boxes;     // device box table, or nullptr: use `one`
     SweepBox one;              // single box passed by value (per-box calls)

@@ -319,32 +319,11 @@ __global__ void box_sums_kernel(int NC, const FabDev* __restrict__ fabs, const P
 
 // ---------------------------------------------------------------- dt
 // estTimeStep (Source/AmrLevelAdv.cpp:395-477 -> FluidSystem.cpp:194-206):
-// cfl * min_d dx_d / max_speed, then the stop-time clamp of
-// computeInitialDt / computeNewDt (Source/AmrLevelAdv.cpp:513-523, 600-611).
 __global__ void step_dt_kernel(StepScalars* s, int D, double dx0, double dx1, double dx2, double cfl, int mode)
 {
     if (s->done) return;
-    if (mode == 1) {
-        s->time = s->time + s->dt;
-        s->steps += 1;
-    }
-    const double ms = __longlong_as_double((long long)s->ws_bits);
-    double dt_est = 1.0e20;
     const double dxs[3] = { dx0, dx1, dx2 };
-    for (int d = 0; d < D; ++d) dt_est = fmin(dt_est, dxs[d] / ms);
-    dt_est *= cfl;
-    double dt_0 = dt_est;
-    if (s->stop_time >= 0.0) {
-        const double eps = 0.001 * dt_0;
-        if ((s->time + dt_0) > (s->stop_time - eps)) dt_0 = s->stop_time - s->time;
-        if (!(s->time < s->stop_time)) s->done = 1;
-    }
-    if (!(dt_est > 0.0) || dt_est != dt_est || isinf(dt_est)) {
-        s->status = 3; /* BAMREX_ERR_NAN */
-        s->done = 1;
-    }
-    s->dt = dt_0;
-    s->ws_bits = 0ull;
+    next_step_scalars(*s, D, dxs, cfl, mode == 1);
 }
 
 // ---------------------------------------------------------------- LR flux

@@ -142,6 +142,23 @@ cudaError_t launch_box_sums(int NC, bool fp32, const FabDev* fabs, const PackBox
 cudaError_t launch_step_dt(StepScalars* scal, int D, double dx0, double dx1, double dx2, double cfl, int mode,
                            cudaStream_t s);
 
+// A run of steps of one short 1D box in one block (line_run.cu): in / out the
+// fab of the starting parity and the other one, cell 0 the box's first.
+struct LineArgs {
+    void* in;
+    void* out;
+    long long in_ns, out_ns;
+    int n, nsteps;
+    bool init;                    // first steps of a run: time and stop_time from here, dt from the state
+    double time, stop_time;
+    double dx, cfl;
+    int bc_lo, bc_hi;             // BAMREX_BC_*
+    StepScalars* scal;
+    Consts k;
+};
+bool line_run_supported(int n);
+cudaError_t launch_line_run(int method, bool fp32, const LineArgs& a, cudaStream_t s);
+
 cudaError_t launch_flux_LR(int D, int dir, int kind, const int* lo, const int* hi, const FabDev& flux,
                            const FabDev& cL, const FabDev& cR, const Consts& k, double dx, double dt,
                            cudaStream_t s);

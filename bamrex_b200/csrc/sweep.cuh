@@ -60,6 +60,15 @@ struct StepFactors {
 };
 
 template <typename T>
+__device__ __forceinline__ void step_factors(double dt, double dx, StepFactors<T>& s)
+{
+    s.dtdx = (T)(dt / dx);               // (dt / dx[d]), AmrLevelAdv_advance.cpp:337
+    s.hdtdx = (T)(0.5 * dt / dx);        // Flux_Helpers.cpp:138
+    s.half_dx_dt = (T)(0.5 * dx / dt);   // Force.cpp:77, 144
+    s.dt_2dx = (T)(dt / (2 * dx));       // Force.cpp:91
+}
+
+template <typename T>
 __device__ __forceinline__ bool step_factors(const SweepArgs& a, StepFactors<T>& s)
 {
     double dt = a.dt_host;
@@ -67,10 +76,7 @@ __device__ __forceinline__ bool step_factors(const SweepArgs& a, StepFactors<T>&
         if (a.scal->done) return false;
         dt = a.scal->dt;
     }
-    s.dtdx = (T)(dt / a.dx);               // (dt / dx[d]), AmrLevelAdv_advance.cpp:337
-    s.hdtdx = (T)(0.5 * dt / a.dx);        // Flux_Helpers.cpp:138
-    s.half_dx_dt = (T)(0.5 * a.dx / dt);   // Force.cpp:77, 144
-    s.dt_2dx = (T)(dt / (2 * a.dx));       // Force.cpp:91
+    step_factors(dt, a.dx, s);
     return true;
 }
 
