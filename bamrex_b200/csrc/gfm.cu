@@ -594,12 +594,13 @@ __global__ void __launch_bounds__(kSweepCta) extrap_kernel(const int* __restrict
 // the storage type T (every update is rounded to T as the state is), the
 // neighbour choice and weights of each swept cell come precomputed, and
 // each thread walks one pencil along x, taking the cell of its pencil on
-// the current plane.  The weights of the next plane's cell are loaded
-// before the barrier so that the plane's critical path is the shared-memory
-// reads, the quotient and the barrier.
+// the current plane.
 
 constexpr int kSmemMax = 224 * 1024;  // shared memory of one (box, component) sweep CTA
-constexpr int kPencilMax = 1024;      // pencils (= threads) of one CTA
+constexpr int kPencilMax = 1024;      // pencils of one CTA, a thread each
+constexpr int kResidentPencils = 512; // the same with all records in shared memory (128 registers a thread)
+constexpr int kLagWarps = 4, kLagPlanes = 8;  // sweeping warps that run one behind the other, and by how much
+constexpr int kSweepHelpers = 256;    // least threads of one CTA, to load and store the region
 
 // Sweep metadata of a swept-region cell, one 16-byte aligned record of
 // rec_words<D>() doubles: w_d = |n_d / dx_d| with the sign giving the
@@ -723,13 +724,177 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // Shared memory of a sweep CTA: the region's values with their halo, then
-// each thread's ring of K metadata records.
-__host__ __device__ inline size_t sweep_smem_bytes(long long hvol, size_t esize, int threads, int K, int rec_bytes)
+// the region's metadata records (K = 0: all `vol` of them) or each sweeping
+// thread's ring of K records.
+__host__ __device__ inline size_t sweep_values_bytes(long long hvol, size_t esize) { return ((size_t)hvol * esize + 15) / 16 * 16; }
+
+// 1D and 2D regions (K = 0: all records in shared memory, 4: a ring of four
+// per thread): one thread per pencil; the other warps of the block help to
+// load and store.  A sweep is a chain of planes (127 of a 64^2
+// region, 8 sweeps a call), so the time is the chain through one plane: the
+// neighbours' values from shared memory (54 cycles with the address), the
+// quotient (six dependent FP64 operations, 115) and the store.  Everything
+// else is off it:
+//  * the record and the addresses of plane t + 1 are in registers before
+//    plane t is stored, from the region's records in shared memory, or from
+//    a ring of the thread's own that cp.async fills K - 1 planes ahead;
+//  * pencils only wait for pencils of lower number (in sweep order) and only
+//    read old values of higher ones, so with K = 0 up to kLagWarps warps run
+//    each kLagPlanes planes behind the warp before, with a barrier every
+//    kLagPlanes planes instead of each one (90 cycles).  More warps spend
+//    longer starting up than that saves; behind a ring the records' copies
+//    are what a plane waits for, and the lag only adds to them (regions of
+//    128^2 1191 -> 1291 us).
+// Not in 3D, where the records' copies are the bound and this only delays
+// them (regions of up to 30^3: 3020 us behind extrap_smem_kernel's ring, 3180 -
+// 4000 in forms of this one), nor behind a ring of two, which would leave no
+// plane in flight.
+// Measured, three calls (24 sweeps) of 64^2 regions with the ghost copies
+// between: 871 us with records and addresses fetched on the chain, 600 with
+// a barrier per plane, 507 now (4 planes of lag 537, 16 the same);
+// regions of 128^2 (K = 4) 1349 -> 1129.
+template <typename T, int D, int K>
+__global__ void __launch_bounds__(K == 0 ? kResidentPencils : kPencilMax) extrap_chain_kernel(const int* __restrict__ list, const int* __restrict__ bbox,
+                                   const long long* __restrict__ meta_off, const double* __restrict__ wts,
+                                   const FabDev* __restrict__ fab_tab, const StepScalars* gate)
 {
-    return (((size_t)hvol * esize + 15) / 16 * 16) + (size_t)threads * K * rec_bytes;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T* sv = reinterpret_cast<T*>(smem_raw);
+    constexpr int NORD = D == 1 ? 2 : (D == 2 ? 4 : 8);
+    constexpr int RW = rec_words<D>();
+    if (gate && gate->done) return;
+    const int li = blockIdx.x, m = blockIdx.y;
+    const int b = list[li];
+    SweepRegion<D> R;
+    R.init(bbox + 6 * b);
+    const double* wt = wts + meta_off[li] * RW;
+    double* recs = reinterpret_cast<double*>(smem_raw + sweep_values_bytes(R.hvol, sizeof(T)));
+    const FabDev f = fab_tab[b];
+    T* u = f.ptr<T>() + m * f.ns;
+    static_assert(D < 3 && (K == 0 || K >= 4), "see above");
+    if constexpr (K == 0) {
+        for (int w = 2 * threadIdx.x; w < R.vol * RW; w += 2 * blockDim.x) cp_async16(recs + w, wt + w);
+        cp_async_group();
+    }
+    region_load<T, D>(R, f, u, sv);
+    if constexpr (K == 0) cp_async_wait<0>();
+    __syncthreads();
+    const int pencils = R.n[1] * R.n[2];
+    const int q = threadIdx.x;
+    const int sweepers = (pencils + 31) / 32 * 32;
+    if (q < sweepers) {
+        double* ring = recs + (size_t)q * K * RW;
+        const bool has = q < pencils;
+        const int pj = has ? q % R.n[1] : 0, pk = has ? q / R.n[1] : 0;
+        const int t0 = pj + pk;  // the plane of this thread's first cell
+        const int planes = R.n[0] + R.n[1] + R.n[2] - 2;
+        // warps 0 .. of the sweep, `lag` rounds of `step` planes behind the first
+        const int nw = sweepers / 32;
+        const int step = nw <= kLagWarps ? kLagPlanes : 1, lag = nw <= kLagWarps ? q / 32 : 0;
+        const int rounds = (planes + step - 1) / step + (nw <= kLagWarps ? nw - 1 : 0);
+        auto on_pencil = [&](int t) { return has && (unsigned)(t - t0) < (unsigned)R.n[0]; };
+        for (int so = 0; so < 2 * NORD; ++so) {
+            int s0, s1, s2;
+            sweep_signs(D, so % NORD, s0, s1, s2);
+            const int cj = s1 > 0 ? pj : R.n[1] - 1 - pj;
+            const int ck = s2 > 0 ? pk : R.n[2] - 1 - pk;
+            const int ci0 = s0 > 0 ? 0 : R.n[0] - 1;
+            // cell of plane t = t0 + e: x = ci0 + s0 e; record r0 + s0 e, smem cs0 + s0 e
+            const int r0 = ci0 + R.n[0] * (cj + R.n[1] * ck);
+            const int cs0 = R.sidx(ci0, cj, ck);
+            // the cell of a plane, with its record: where it is, which
+            // neighbours it takes; `on` is false off the pencil and for a
+            // cell the sweeps skip
+            struct Next {
+                double rec[RW];
+                bool on;
+                int cs, nb[3];
+            } nxt;
+            auto issue = [&](int t) {
+                if constexpr (K > 1) {
+                    // (an empty group off the pencil keeps one group per plane)
+                    if (on_pencil(t)) {
+                        const double* src = wt + (long long)(r0 + s0 * (t - t0)) * RW;
+                        double* dst = ring + (t % K) * RW;
+#pragma unroll
+                        for (int w = 0; w < RW; w += 2) cp_async16(dst + w, src + w);
+                    }
+                    cp_async_group();
+                }
+            };
+            auto fetch = [&](int t) {
+                const int e = min(max(t - t0, 0), R.n[0] - 1);
+                const double* src = K == 0 ? recs + (r0 + s0 * e) * RW : ring + (t % K) * RW;
+#pragma unroll
+                for (int w = 0; w < RW; w += 2) {
+                    const double2 v = *reinterpret_cast<const double2*>(src + w);
+                    nxt.rec[w] = v.x;
+                    nxt.rec[w + 1] = v.y;
+                }
+                nxt.on = on_pencil(t) && nxt.rec[D] >= 0;
+                nxt.cs = cs0 + s0 * e;
+                nxt.nb[0] = nxt.cs + (signbit(nxt.rec[0]) ? -1 : 1);
+                if (D > 1) nxt.nb[1] = nxt.cs + (signbit(nxt.rec[1]) ? -R.so1 : R.so1);
+                if (D > 2) nxt.nb[2] = nxt.cs + (signbit(nxt.rec[2]) ? -R.so2 : R.so2);
+            };
+            auto neighbours = [&](const Next& c, double (&v)[D]) {
+#pragma unroll
+                for (int d = 0; d < D; ++d) v[d] = (double)sv[c.nb[d]];
+            };
+            auto update = [&](const Next& c, const double (&v)[D]) {
+                double num = 0.0 + fabs(c.rec[0]) * v[0];
+#pragma unroll
+                for (int d = 1; d < D; ++d) num = num + fabs(c.rec[d]) * v[d];
+                const T val = (T)div_by_rcp(num, c.rec[D], c.rec[D + 1]);
+                if (c.on) sv[c.cs] = val;
+            };
+            auto barrier = [&] { asm volatile("bar.sync 1, %0;" ::"r"(sweepers) : "memory"); };
+#pragma unroll
+            for (int t = 0; t < K - 1; ++t) issue(t);
+            if constexpr (K > 1) cp_async_wait<K - 2>();
+            fetch(0);
+            auto plane = [&](int t) {
+                const Next c = nxt;
+                double v[D];
+                neighbours(c, v);
+                if constexpr (K > 1) {
+                    issue(t + K - 1);
+                    cp_async_wait<K - 2>();
+                }
+                fetch(t + 1);
+                update(c, v);
+            };
+            if constexpr (K == 0) {
+                for (int round = 0; round < rounds; ++round) {
+                    const int tb = (round - lag) * step, te = min(tb + step, planes);
+                    for (int t = max(tb, 0); t < te; ++t) {
+                        plane(t);
+                        __syncwarp();
+                    }
+                    barrier();
+                }
+            } else {
+                for (int t = 0; t < planes; ++t) {
+                    plane(t);
+                    barrier();
+                }
+            }
+            if constexpr (K > 1) cp_async_wait<0>();
+        }
+    }
+    __syncthreads();
+    // swept cells back to the state
+#pragma unroll 4
+    for (int r = threadIdx.x; r < R.vol; r += blockDim.x) {
+        if (!((K == 0 ? recs : wt)[(long long)r * RW + D] >= 0)) continue;
+        const int ci = r % R.n[0], rr = r / R.n[0];
+        const int cj = rr % R.n[1], ck = rr / R.n[1];
+        u[at(f, R.lo[0] + ci, R.lo[1] + cj, R.lo[2] + ck)] = sv[R.sidx(ci, cj, ck)];
+    }
 }
 
-// One thread per pencil (up to 1024 pencils), a barrier per plane.  Each
+// 3D regions, and 2D ones without room for four records per thread: one
+// thread per pencil (up to 1024 pencils), a barrier per plane.  Each
 // thread streams the metadata record of its cell K - 1 planes ahead into a
 // ring of its own in shared memory (cp.async), so the plane's critical path
 // is the shared-memory reads, the quotient and the barrier; K = 1 (no room
@@ -749,7 +914,7 @@ __global__ void __launch_bounds__(kPencilMax) extrap_smem_kernel(const int* __re
     SweepRegion<D> R;
     R.init(bbox + 6 * b);
     const double* wt = wts + meta_off[li] * RW;
-    double* ring = reinterpret_cast<double*>(smem_raw + ((size_t)R.hvol * sizeof(T) + 15) / 16 * 16) +
+    double* ring = reinterpret_cast<double*>(smem_raw + sweep_values_bytes(R.hvol, sizeof(T))) +
                    (size_t)threadIdx.x * K * RW;
     const FabDev f = fab_tab[b];
     T* u = f.ptr<T>() + m * f.ns;
@@ -1006,6 +1171,14 @@ Sdf make_sdf(const bamrex_sdf& s)
 
 int body_launch(bamrex_level* L, cudaError_t e, const char* what) { return level_launch(L, e, what); }
 
+// The kernel of a level's regions for its number of records in flight.
+template <typename T, int D, int K>
+auto sweep_kernel()
+{
+    if constexpr (D < 3 && (K == 0 || K == 4)) return extrap_chain_kernel<T, D, K>;
+    else return extrap_smem_kernel<T, D, K == 0 ? 1 : K>;  // (K = 0 is not set in 3D)
+}
+
 // The dynamic shared-memory limit of the sweep kernel: a property of the
 // kernel, shared by every level that uses it, so it is raised to the most
 // any level may ask (kSmemMax) rather than to this level's need (a level
@@ -1017,13 +1190,13 @@ cudaError_t smem_attribute(bool fp32, int D, int bytes)
     bytes = kSmemMax;
     const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
     if (fp32) {
-        if (D == 1) return cudaFuncSetAttribute(extrap_smem_kernel<float, 1, K>, a, bytes);
-        if (D == 2) return cudaFuncSetAttribute(extrap_smem_kernel<float, 2, K>, a, bytes);
-        return cudaFuncSetAttribute(extrap_smem_kernel<float, 3, K>, a, bytes);
+        if (D == 1) return cudaFuncSetAttribute(sweep_kernel<float, 1, K>(), a, bytes);
+        if (D == 2) return cudaFuncSetAttribute(sweep_kernel<float, 2, K>(), a, bytes);
+        return cudaFuncSetAttribute(sweep_kernel<float, 3, K>(), a, bytes);
     }
-    if (D == 1) return cudaFuncSetAttribute(extrap_smem_kernel<double, 1, K>, a, bytes);
-    if (D == 2) return cudaFuncSetAttribute(extrap_smem_kernel<double, 2, K>, a, bytes);
-    return cudaFuncSetAttribute(extrap_smem_kernel<double, 3, K>, a, bytes);
+    if (D == 1) return cudaFuncSetAttribute(sweep_kernel<double, 1, K>(), a, bytes);
+    if (D == 2) return cudaFuncSetAttribute(sweep_kernel<double, 2, K>(), a, bytes);
+    return cudaFuncSetAttribute(sweep_kernel<double, 3, K>(), a, bytes);
 }
 
 int ghost_ops(bamrex_level* L, const GhostOp* ops, int nops, int nchunks, int parity, const StepScalars* gate)
@@ -1097,10 +1270,11 @@ int body_fill(bamrex_level* L, int parity, const StepScalars* gate)
         if (S->n_smem) {
             const dim3 g((unsigned)S->n_smem, (unsigned)L->NC);
 #define BX_EXTRAP_S(T, DD, KK)                                                                               \
-    extrap_smem_kernel<T, DD, KK><<<g, S->threads_p, S->bytes_p, L->stream>>>(S->d_list_s, S->d_bbox, S->d_meta_off, \
+    sweep_kernel<T, DD, KK>()<<<g, S->threads_p, S->bytes_p, L->stream>>>(S->d_list_s, S->d_bbox, S->d_meta_off, \
                                                                               S->d_wts, L->d_fab[parity], gate)
 #define BX_EXTRAP_SK(T, DD) \
-    if (S->ring == 4) BX_EXTRAP_S(T, DD, 4); else if (S->ring == 2) BX_EXTRAP_S(T, DD, 2); else BX_EXTRAP_S(T, DD, 1)
+    if (S->ring == 0) BX_EXTRAP_S(T, DD, 0); else if (S->ring == 4) BX_EXTRAP_S(T, DD, 4); \
+    else if (S->ring == 2) BX_EXTRAP_S(T, DD, 2); else BX_EXTRAP_S(T, DD, 1)
             if (L->fp32) {
                 if (D == 1) { BX_EXTRAP_SK(float, 1); }
                 else if (D == 2) { BX_EXTRAP_SK(float, 2); }
@@ -1266,8 +1440,8 @@ extern "C" int bamrex_level_set_body(bamrex_level* L, const bamrex_body_desc* de
     // fit (one CTA per box and component), else the global-memory kernel
     std::vector<int> list_p, list_g;
     std::vector<long long> vol_p;
-    size_t bytes_p = 0;
-    int threads_p = 32;
+    size_t bytes_p = 0, resident_p = 0;  // values alone; with every record
+    int threads_p = D < 3 ? kSweepHelpers : 32, pencils_p = 32;
     const int rec_bytes = 8 * (D == 1 ? rec_words<1>() : (D == 2 ? rec_words<2>() : rec_words<3>()));
     for (int b = 0; b < nb; ++b) {
         if (bbox[6 * b] > bbox[6 * b + 3]) continue;
@@ -1279,25 +1453,33 @@ extern "C" int bamrex_level_set_body(bamrex_level* L, const bamrex_body_desc* de
         }
         const long long pencils = n[1] * n[2];
         // the region's values (a ring comes on top only where it fits)
-        const size_t values = sweep_smem_bytes(hv, L->esize, 0, 1, rec_bytes);
+        const size_t values = sweep_values_bytes(hv, L->esize);
         if (pencils > kPencilMax || values > (size_t)kSmemMax) {
             list_g.push_back(b);
         } else {
             list_p.push_back(b);
             vol_p.push_back(vol);
             bytes_p = std::max(bytes_p, values);
+            resident_p = std::max(resident_p, values + (size_t)(vol * rec_bytes));
+            pencils_p = std::max(pencils_p, (int)((pencils + 31) / 32 * 32));
             threads_p = std::max(threads_p, (int)((pencils + 31) / 32 * 32));
         }
     }
-    // the deepest ring (records in flight per thread) that fits
+    // all records in shared memory, else the deepest ring (records in flight
+    // per thread) that fits
     int ring = 1;
-    for (int K : { 4, 2 })
-        if (bytes_p + (size_t)threads_p * K * rec_bytes <= (size_t)kSmemMax) {
-            ring = K;
-            break;
-        }
+    if (D < 3 && resident_p <= (size_t)kSmemMax && pencils_p <= kResidentPencils) {
+        ring = 0;
+        bytes_p = resident_p;
+    } else {
+        for (int K : { 4, 2 })
+            if (bytes_p + (size_t)pencils_p * K * rec_bytes <= (size_t)kSmemMax) {
+                ring = K;
+                bytes_p += (size_t)pencils_p * K * rec_bytes;
+                break;
+            }
+    }
     S->ring = ring;
-    bytes_p += ring > 1 ? (size_t)threads_p * ring * rec_bytes : 0;
     const std::vector<int>& list_s = list_p;
     std::vector<long long> meta_off;
     long long meta_cells = 0;
@@ -1353,7 +1535,7 @@ extern "C" int bamrex_level_set_body(bamrex_level* L, const bamrex_body_desc* de
         e = cudaGetLastError();
         L->launches++;
         if (e == cudaSuccess)
-            e = ring == 4 ? smem_attribute<4>(L->fp32, D, (int)bytes_p)
+            e = ring == 0 ? smem_attribute<0>(L->fp32, D, (int)bytes_p) : ring == 4 ? smem_attribute<4>(L->fp32, D, (int)bytes_p)
                           : (ring == 2 ? smem_attribute<2>(L->fp32, D, (int)bytes_p) : smem_attribute<1>(L->fp32, D, (int)bytes_p));
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(L->stream);
