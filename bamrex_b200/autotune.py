@@ -1,6 +1,6 @@
 """Autotuner for the sweep launches of a level: per direction the sweep
-kernel (how it stages its input and shares the stencil: the L2-loading row
-or marching kernels, the TMA-staged per-warp march, or the TMA-staged block
+kernel (how it stages its input and shares the stencil: the row-group or
+marching register kernels, the TMA-staged per-warp march, or the TMA-staged block
 wavefront) and then the work-item shape (segment lengths along the sweep)
 are chosen by timing the candidates on the device with the level's own
 sweep timing events, and remembered per configuration (device, dimension,
@@ -23,7 +23,7 @@ from . import _abi
 X_CANDIDATES = (32, 64, 128, 256, 512, 1024, 2048)
 S_CANDIDATES = (16, 24, 32, 48, 64, 96, 128, 256)
 # (staging, x_mode) of each kernel kind tried; x_mode only matters for the
-# L2-loading x sweep
+# register x sweep
 KINDS = {"rows": (_abi.STAGING_REGISTERS, _abi.XSWEEP_ROWS), "march": (_abi.STAGING_REGISTERS, _abi.XSWEEP_MARCH),
          "tma": (_abi.STAGING_TMA, _abi.XSWEEP_AUTO), "wave": (_abi.STAGING_WAVE, _abi.XSWEEP_AUTO)}
 _CACHE_VERSION = 2

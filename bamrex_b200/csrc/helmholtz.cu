@@ -15,7 +15,10 @@
 // the boundary value cf * x(cell) with cf = +1 (homogeneous Neumann) or -1
 // (homogeneous Dirichlet on the face); the smoother moves the cf part to the
 // left-hand side as the reference's cf/delta terms do.  Every kernel is
-// HBM-bound; this file is compiled with -fmad=false so each operation rounds
+// HBM-bound, or bound by latency on the way to it; in 2D half a level of the
+// V-cycle is one launch over tiles (helmholtz_tile.cuh), the coarse levels one
+// block (helmholtz_small.cuh), and BiCGStab's dot products are taken by the
+// kernels that make their vectors.  This file is compiled with -fmad=false so each operation rounds
 // exactly as written and a CPU restatement reproduces apply and smooth bit
 // for bit.
 #include <cuda_runtime.h>

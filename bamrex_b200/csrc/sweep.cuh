@@ -12,6 +12,8 @@
 //    columns x and a segment along the sweep; each thread marches its column
 //    keeping the stencil in registers.  Loads and stores are coalesced
 //    across the warp (32 consecutive values per component).
+// These kernels run the y / z sweeps of the general path (the fast path's are
+// TMA-staged, sweep_tma.cuh) and the x sweeps of levels of narrow boxes.
 // The march is software-pipelined: the face stage of an iteration uses cell
 // stages finished in earlier iterations, so the cell stage (reconstruction
 // + half step) and the face stage (Riemann flux) of one iteration are

@@ -93,7 +93,7 @@ def sweep_kernel_name(D, d, kind, x_rows):
         return "sweep_wave_kernel<%d,%d>" % (D, d)
     if kind == 2:
         return "sweep_tma_kernel<%d,%d>" % (D, d)
-    return "sweep_x_kernel<%d>" % D if (d == 0 and x_rows) else "sweep_s_kernel<%d,%d>" % (D, d)
+    return "sweep_row_kernel<%d>" % D if (d == 0 and x_rows) else "sweep_s_kernel<%d,%d>" % (D, d)
 
 
 def parity_check(lev, u_start, n, steps_from):
