@@ -190,29 +190,46 @@ void box_items(int dir, const int* lo, const int* hi, int seglen, long long& ite
 // large ones long segments.
 int choose_seglen(int dir, const std::vector<bamrex_box>& boxes, long long resident_warps, bool march = false)
 {
-    std::vector<int> cand = { 256, 192, 128, 96, 64, 48, 32, 24, 16, 12, 8 };
+    if (dir == 0 && !march) return 256;  // row groups take whole rows
+    // a box's cells along dir and its lane groups (the same for every length)
+    struct Line {
+        int n, ngroup;
+    };
+    Line first;
+    std::vector<Line> more;  // of a level's further boxes: a per-box call allocates nothing
     int nmax = 1;
-    for (const auto& b : boxes) nmax = std::max(nmax, b.hi[dir] - b.lo[dir] + 1);
-    for (int m = 1; m <= 24; ++m)
-        if ((nmax + m - 1) / m >= 4) cand.push_back(std::min(256, (nmax + m - 1) / m));
+    for (size_t i = 0; i < boxes.size(); ++i) {
+        const auto& b = boxes[i];
+        Line l;
+        l.n = b.hi[dir] - b.lo[dir] + 1;
+        long long it;
+        int nseg;
+        box_items(dir, b.lo, b.hi, l.n, it, nseg, l.ngroup, march);
+        nmax = std::max(nmax, l.n);
+        if (i == 0) first = l;
+        else more.push_back(l);
+    }
     const long long W = std::max(1LL, resident_warps);
     int best = 64;
     double best_time = -1;
-    for (int c : cand) {
+    auto consider = [&](int c) {
         long long items = 0, steps = 0;
-        for (const auto& b : boxes) {
-            long long it;
-            int nseg, ngroup;
-            box_items(dir, b.lo, b.hi, c, it, nseg, ngroup, march);
-            items += it;
-            steps += (long long)ngroup * (b.hi[dir] - b.lo[dir] + 1 + 5LL * nseg);
-        }
+        auto add = [&](const Line& l) {
+            const int nseg = (l.n + c - 1) / c;
+            items += (long long)l.ngroup * nseg;
+            steps += (long long)l.ngroup * (l.n + 5LL * nseg);
+        };
+        add(first);
+        for (const Line& l : more) add(l);
         const double t = (double)((items + W - 1) / W) * (double)steps / (double)items;
         if (best_time < 0 || t < best_time) {
             best = c;
             best_time = t;
         }
-    }
+    };
+    for (int c : { 256, 192, 128, 96, 64, 48, 32, 24, 16, 12, 8 })
+        if (c == 256 || c < nmax) consider(c);  // longer than every line: one segment, as 256
+    for (int m = 1; m <= 24 && (nmax + m - 1) / m >= 4; ++m) consider(std::min(256, (nmax + m - 1) / m));
     return best;
 }
 
