@@ -725,7 +725,7 @@ __device__ __forceinline__ void hllc_face_f64(const double (&L)[D + 2], const do
 }
 
 // |u| + c, within a few ulp; NaN for a negative pressure or density, as the
-// roots are.  Both radicands are offset by 1e-300: exact for every normal
+// roots are, and infinite where a square is.  Both radicands are offset by 1e-300: exact for every normal
 // value above 1e-284, and a fluid at rest (or without pressure) adds 1e-150
 // instead of 0, which the sum's rounding drops unless both vanish (reduce_ws
 // takes such a maximum back to 0).
@@ -736,7 +736,12 @@ __device__ __forceinline__ double wave_speed_f64(const double (&U)[D + 2], const
     double mu = q.mnu;
 #pragma unroll
     for (int d = 1; d < D; ++d) mu = fma(U[1 + d], q.u[d], mu);
-    return sqrt_pos(fma(k.gamma_inv_eps * q.p, q.ir, 1e-300)) + sqrt_pos(fma(mu, q.ir, 1e-300));
+    const double c2 = fma(k.gamma_inv_eps * q.p, q.ir, 1e-300), v2 = fma(mu, q.ir, 1e-300);
+    auto root = [](double x) {
+        const double r = sqrt_pos(x);
+        return __double2hiint(x) == 0x7ff00000 ? x : r;  // (the maximum keeps an infinity)
+    };
+    return root(c2) + root(v2);
 }
 
 // ---- FP32 storage: the same scheme with the hardware approximations -------

@@ -41,11 +41,11 @@ __device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long v
     return ((unsigned long long)top << 32) | low;
 }
 
-// A NaN or infinity as the NaN pattern, above every finite value.
+// A NaN as the NaN pattern, above every other value.
 template <typename T>
 __device__ __forceinline__ unsigned long long speed_bits(const WsMax<T>& w)
 {
-    if (w.bad()) return 0x7ff8000000000000ull;
+    if (w.nan()) return 0x7ff8000000000000ull;
     const double v = (double)w.v;
     return v < 1e-140 ? 0ull : (unsigned long long)__double_as_longlong(v);  // wave_speed_f64's offset
 }

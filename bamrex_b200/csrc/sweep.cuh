@@ -108,9 +108,9 @@ __device__ __forceinline__ void copy_state(const T (&s)[NC], T (&d)[NC])
 }
 
 // The running maximum of the wave speed |u| + c of a thread's updated cells,
-// in the kernel's own type, without a branch: the value by one comparison,
-// and the largest exponent field beside it (NaN and infinity show there; the
-// comparison alone would drop a NaN).
+// in the kernel's own type, without a branch: the value by one comparison
+// (which keeps an infinity), and the largest high word beside it, where a NaN
+// shows (the comparison alone would drop it).
 template <typename T>
 struct WsMax {
     T v = T(0);
@@ -123,24 +123,23 @@ struct WsMax {
         v = w > v ? w : v;
         top = max(top, bits(w));
     }
-    __device__ __forceinline__ bool bad() const { return top >= (sizeof(T) == 8 ? 0x7ff00000 : 0x7f800000); }
+    __device__ __forceinline__ bool nan() const { return top > (sizeof(T) == 8 ? 0x7ff00000 : 0x7f800000); }
 };
 
 // Warp max of the wave speed, then one atomicMax per warp on the ordered bit
-// pattern (non-negative doubles order like their bits).  A NaN or infinity
-// anywhere is reported as the NaN bit pattern, which is larger than every
-// finite value, so the time step becomes NaN and the host sees
-// BAMREX_ERR_NAN.
+// pattern (non-negative doubles order like their bits).  An infinity makes the
+// time step zero, which ends a run or an estimate with BAMREX_ERR_NAN.  A NaN
+// anywhere is reported as the NaN bit pattern, above every other value.
 template <typename T>
 __device__ __forceinline__ void reduce_ws(const WsMax<T>& w, unsigned long long* dst)
 {
     double ws = (double)w.v;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) ws = fmax(ws, __shfl_xor_sync(0xffffffffu, ws, off));
-    const bool any_bad = __any_sync(0xffffffffu, w.bad());
+    const bool any_nan = __any_sync(0xffffffffu, w.nan());
     if (ws < 1e-140) ws = 0.0;  // wave_speed_f64's offset of a state without pressure and motion
     if ((threadIdx.x & 31) == 0) {
-        if (any_bad) atomicMax(dst, 0x7ff8000000000000ull);
+        if (any_nan) atomicMax(dst, 0x7ff8000000000000ull);
         else if (ws > 0.0) atomicMax(dst, (unsigned long long)__double_as_longlong(ws));
     }
 }
