@@ -209,9 +209,13 @@ cudaError_t launch_line_run(int method, bool fp32, const LineArgs& a, cudaStream
     const int lim = fast_limiter(1, method, a.k);
     const void* fn = fp32 ? pick_line_kernel<float>(method, lim) : pick_line_kernel<double>(method, lim);
     if (!fn) return cudaErrorInvalidValue;
-    const size_t smem = 2 * 3 * (size_t)(a.n + 2 * kLineGhost) * (fp32 ? sizeof(float) : sizeof(double));
+    const auto line_bytes = [fp32](int n) { return 2 * 3 * (size_t)(n + 2 * kLineGhost) * (fp32 ? sizeof(float) : sizeof(double)); };
+    const size_t smem = line_bytes(a.n);
     if (smem > 40 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // the limit is the kernel's, shared by every level and thread that
+        // uses it: always the longest line's, so that no launch lowers it
+        // under another's
+        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)line_bytes(kLineMaxCells));
         if (e != cudaSuccess) return e;
     }
     const int chunks = (a.n + kLineOwned - 1) / kLineOwned;
