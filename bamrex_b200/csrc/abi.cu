@@ -531,7 +531,7 @@ static int per_box_sweep(int method, int dir, int D, const bamrex_box* bx, const
     const std::vector<bamrex_box> one(1, *bx);
     a.seglen = dir == 0 ? bx->hi[0] - bx->lo[0] + 1 : choose_seglen(dir, one, sweep_resident_warps(D, dir, method, false, k));
     long long items;
-    box_items(dir, B.lo, B.hi, a.seglen, items, B.nseg, B.ngroup, false, &B.seglen, row_positions(fast_limiter(D, method, k)));
+    box_items(dir, B.lo, B.hi, a.seglen, items, B.nseg, B.ngroup, false, &B.seglen, row_positions(fast_limiter(D, method, false, k)));
     // pairs of the row lie at an even distance from lo: aligned when cell lo
     // and the strides are
     auto paired = [&](const bamrex_array4& f) {
@@ -879,7 +879,7 @@ int level_sweep(bamrex_level* L, int d, int parity, double dt_host, const StepSc
     int rc;
     if (L->tma(d)) {
         a.status = &L->d_scal->status;
-        rc = level_launch(L, launch_sweep_tma(L->D, d, L->fp32, fast_limiter(L->D, L->method, L->k), L->wave(d), a, L->stream),
+        rc = level_launch(L, launch_sweep_tma(L->D, d, L->fp32, fast_limiter(L->D, L->method, L->fp32, L->k), L->wave(d), a, L->stream),
                           "TMA-staged sweep");
     } else {
         rc = level_launch(L, launch_sweep(L->D, d, L->method, L->fp32, a, L->stream, d == 0 && L->x_march), "sweep");
@@ -1058,7 +1058,7 @@ extern "C" int bamrex_level_create(bamrex_level** out, const bamrex_level_desc* 
         return fail(BAMREX_ERR_ARG, "staging must be BAMREX_STAGING_AUTO, _REGISTERS, _TMA or _WAVE");
     }
     {
-        const bool fast = tma_supported(D, L->method, L->k);
+        const bool fast = tma_supported(D, L->method, L->fp32, L->k);
         const bool ok = fast || (D >= 2 && tma_requestable(D, L->method, L->k));
         if ((desc->staging == BAMREX_STAGING_TMA || desc->staging == BAMREX_STAGING_WAVE) && !ok) {
             delete L;
@@ -1093,7 +1093,7 @@ extern "C" int bamrex_level_create(bamrex_level** out, const bamrex_level_desc* 
     auto tma_seg = [&](int d, bool wave) {
         int& m = memo_tma[d][wave ? 1 : 0];
         if (m < 0) {
-            const int lim = fast_limiter(D, L->method, L->k);
+            const int lim = fast_limiter(D, L->method, L->fp32, L->k);
             m = choose_tma_seglen(D, d, L->boxes, sweep_tma_resident_units(D, d, L->fp32, lim, wave), wave);
         }
         return m;
@@ -1101,10 +1101,10 @@ extern "C" int bamrex_level_create(bamrex_level** out, const bamrex_level_desc* 
     std::vector<SweepBox> sweep_host[3];
     // the register kernel of the x sweep when the caller leaves it open
     L->x_march = D >= 2 && (desc->x_mode == BAMREX_XSWEEP_MARCH || (desc->x_mode == BAMREX_XSWEEP_AUTO && narrow_rows(L->boxes)));
-    const int row_p = row_positions(fast_limiter(D, L->method, L->k));
+    const int row_p = row_positions(fast_limiter(D, L->method, L->fp32, L->k));
     for (int d = 0; d < D; ++d) {
         if (L->sweep_kind[d] >= 0) continue;
-        if (!tma_supported(D, L->method, L->k)) {
+        if (!tma_supported(D, L->method, L->fp32, L->k)) {
             L->sweep_kind[d] = BAMREX_STAGING_REGISTERS;
             continue;
         }
@@ -1675,7 +1675,7 @@ int host_step_enqueue(bamrex_level* L, const double* host_in, double* host_out, 
             sa.ws_max = ws ? &L->d_scal->ws_bits : nullptr;
             sa.do_update = 1;
             sa.status = &L->d_scal->status;
-            return level_launch(L, launch_sweep_tma(D, dir, L->fp32, fast_limiter(D, L->method, L->k), L->wave(dir), sa,
+            return level_launch(L, launch_sweep_tma(D, dir, L->fp32, fast_limiter(D, L->method, L->fp32, L->k), L->wave(dir), sa,
                                                     L->stream),
                                 "slab sweep");
         }
@@ -1693,7 +1693,7 @@ int host_step_enqueue(bamrex_level* L, const double* host_in, double* host_out, 
         const bool march = dir == 0 && L->x_march;
         long long items;
         box_items(dir, sb.lo, sb.hi, L->seglen[dir], items, sb.nseg, sb.ngroup, march, &sb.seglen,
-                  row_positions(fast_limiter(D, L->method, L->k)));
+                  row_positions(fast_limiter(D, L->method, L->fp32, L->k)));
         sb.item_begin = 0;
         sa.total_items = items;
         sa.seglen = L->seglen[dir];
@@ -1878,7 +1878,7 @@ extern "C" int bamrex_level_est_time_step(bamrex_level* L, double* dt_est)
     if (!L->ws_valid) {
         cudaError_t e = cudaMemsetAsync(&L->d_scal->ws_bits, 0, sizeof(unsigned long long), L->stream);
         if (e != cudaSuccess) return L->set_err(cuda_fail(e, "memset"));
-        BX_TRY(level_launch(L, launch_max_wave_speed(L->D, L->fp32, fast_limiter(L->D, L->method, L->k) >= 0, L->d_fab[L->cur], L->d_pack, (int)L->boxes.size(), L->ncells, L->k,
+        BX_TRY(level_launch(L, launch_max_wave_speed(L->D, L->fp32, fast_limiter(L->D, L->method, L->fp32, L->k) >= 0, L->d_fab[L->cur], L->d_pack, (int)L->boxes.size(), L->ncells, L->k,
                                                      &L->d_scal->ws_bits, nullptr, L->stream),
                             "max wave speed"));
     }
@@ -1970,7 +1970,7 @@ extern "C" int bamrex_level_run_async(bamrex_level* L, int nsteps, double stop_t
         e = cudaMemcpyAsync(L->d_scal, h, sizeof(StepScalars), cudaMemcpyHostToDevice, L->stream);
         if (e != cudaSuccess) return L->set_err(cuda_fail(e, "scalars upload"));
         // computeInitialDt from the current state
-        BX_TRY(level_launch(L, launch_max_wave_speed(L->D, L->fp32, fast_limiter(L->D, L->method, L->k) >= 0, L->d_fab[L->cur], L->d_pack, (int)L->boxes.size(), L->ncells, L->k,
+        BX_TRY(level_launch(L, launch_max_wave_speed(L->D, L->fp32, fast_limiter(L->D, L->method, L->fp32, L->k) >= 0, L->d_fab[L->cur], L->d_pack, (int)L->boxes.size(), L->ncells, L->k,
                                                      &L->d_scal->ws_bits, L->d_scal, L->stream),
                             "max wave speed"));
         BX_TRY(level_launch(L, launch_step_dt(L->d_scal, L->D, L->dx[0], L->dx[1], L->dx[2], L->cfl, 0, L->stream), "step dt"));

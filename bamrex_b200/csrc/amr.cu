@@ -1915,7 +1915,7 @@ int coarse_step_graph(bamrex_amr* A, double stop_time, double time)
             if (L->ws_valid) continue;
             e = cudaMemsetAsync(&L->d_scal->ws_bits, 0, sizeof(unsigned long long), L->stream);
             if (e == cudaSuccess)
-                e = launch_max_wave_speed(L->D, L->fp32, fast_limiter(L->D, L->method, L->k) >= 0, L->d_fab[L->cur], L->d_pack, (int)L->boxes.size(), L->ncells,
+                e = launch_max_wave_speed(L->D, L->fp32, fast_limiter(L->D, L->method, L->fp32, L->k) >= 0, L->d_fab[L->cur], L->d_pack, (int)L->boxes.size(), L->ncells,
                                           L->k, &L->d_scal->ws_bits, nullptr, L->stream);
             if (e != cudaSuccess) return amr_fail(A, BAMREX_ERR_CUDA, std::string("max wave speed: ") + cudaGetErrorString(e));
             L->launches++;

@@ -16,7 +16,7 @@ cudaError_t launch_register_faces(int D, int dir, int method, bool fp32, const C
                                   const SweepBox* xsw)
 {
     (void)NC;
-    const int lim = fast_limiter(D, method, k);
+    const int lim = fast_limiter(D, method, fp32, k);
     const void* fn = fp32 ? pick_register_kernel<float>(D, dir, method, lim)
                           : pick_register_kernel<double>(D, dir, method, lim);
     if (!fn) return cudaErrorInvalidValue;

@@ -134,7 +134,7 @@ extern "C" int bamrex_level_wave_speed(bamrex_level* L, double* ws)
     if (!L->ws_valid) {
         cudaError_t e = cudaMemsetAsync(&L->d_scal->ws_bits, 0, sizeof(unsigned long long), L->stream);
         if (e != cudaSuccess) return L->set_err(cuda_fail(e, "memset"));
-        BX_TRY(level_launch(L, launch_max_wave_speed(L->D, L->fp32, fast_limiter(L->D, L->method, L->k) >= 0, L->d_fab[L->cur], L->d_pack, (int)L->boxes.size(),
+        BX_TRY(level_launch(L, launch_max_wave_speed(L->D, L->fp32, fast_limiter(L->D, L->method, L->fp32, L->k) >= 0, L->d_fab[L->cur], L->d_pack, (int)L->boxes.size(),
                                                      L->ncells, L->k, &L->d_scal->ws_bits, nullptr, L->stream),
                             "max wave speed"));
     }
@@ -166,7 +166,7 @@ extern "C" int bamrex_level_dist_begin(bamrex_level* L, double time, double stop
     h->stop_time = stop_time;
     cudaError_t e = cudaMemcpyAsync(L->d_scal, h, sizeof(StepScalars), cudaMemcpyHostToDevice, L->stream);
     if (e != cudaSuccess) return L->set_err(cuda_fail(e, "scalars upload"));
-    BX_TRY(level_launch(L, launch_max_wave_speed(L->D, L->fp32, fast_limiter(L->D, L->method, L->k) >= 0, L->d_fab[L->cur], L->d_pack, (int)L->boxes.size(),
+    BX_TRY(level_launch(L, launch_max_wave_speed(L->D, L->fp32, fast_limiter(L->D, L->method, L->fp32, L->k) >= 0, L->d_fab[L->cur], L->d_pack, (int)L->boxes.size(),
                                                  L->ncells, L->k, &L->d_scal->ws_bits, L->d_scal, L->stream),
                         "max wave speed"));
     L->run_pending = true;

@@ -91,9 +91,9 @@ long long sweep_resident_warps(int D, int dir, int method, bool fp32, const Cons
 
 // The fast-path limiter for this configuration (MUSCL-Hancock, energy
 // limiting, gamma with 1/z = 7), or -1 for the general kernels.
-int fast_limiter(int D, int method, const Consts& k);
+int fast_limiter(int D, int method, bool fp32, const Consts& k);
 // Whether a level may ask for the TMA-staged kernels: the fast path's
-// configurations, and a gamma that misses 1/z = 7 by more than its own
+// configurations, and in FP64 a gamma that misses 1/z = 7 by more than its own
 // rounding but by less than 1e-12, for which the request runs the general
 // register kernels.
 bool tma_requestable(int D, int method, const Consts& k);
@@ -107,7 +107,7 @@ bool tma_requestable(int D, int method, const Consts& k);
 // 256-byte aligned start of the fab's first padded row); the launch runs
 // over a level's box table (boxes carry tmap, wa, xoff).  Resident units:
 // warps (march) or blocks (wavefront).
-bool tma_supported(int D, int method, const Consts& k);
+bool tma_supported(int D, int method, bool fp32, const Consts& k);
 int tma_item_lines(bool wave, int dir);
 int tma_pass_positions(bool wave, int dir);
 cudaError_t encode_sweep_tmap(void* out, bool fp32, int D, int NC, int dir, bool wave, int wa, const void* row_start,

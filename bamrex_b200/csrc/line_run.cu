@@ -206,7 +206,7 @@ bool line_run_supported(int n) { return n >= 2 * kLineGhost && n <= kLineMaxCell
 
 cudaError_t launch_line_run(int method, bool fp32, const LineArgs& a, cudaStream_t s)
 {
-    const int lim = fast_limiter(1, method, a.k);
+    const int lim = fast_limiter(1, method, fp32, a.k);
     const void* fn = fp32 ? pick_line_kernel<float>(method, lim) : pick_line_kernel<double>(method, lim);
     if (!fn) return cudaErrorInvalidValue;
     const auto line_bytes = [fp32](int n) { return 2 * 3 * (size_t)(n + 2 * kLineGhost) * (fp32 ? sizeof(float) : sizeof(double)); };

@@ -51,13 +51,14 @@ int blocks_per_sm(const void* fn, int smem)
 
 }  // namespace
 
-// The fast path takes 1/z = 7 exactly.  The rounding of gamma = 1.4 (an ulp
-// or two either way) leaves |1/z - 7| below 1e-14, whose effect on the
+// The fast path takes 1/z = 7 exactly in FP64.  The rounding of gamma = 1.4 (an
+// ulp or two either way) leaves |1/z - 7| below 1e-14, whose effect on the
 // two-rarefaction pressure, (1/z - 7) ln b, is within the rounding of b^7;
-// a gamma further off runs the general kernels, which correct for it.
-int fast_limiter(int D, int method, const Consts& k)
+// a gamma further off runs the general kernels, which correct for it.  FP32
+// storage takes 1/z as it is (exponential and logarithm).
+int fast_limiter(int D, int method, bool fp32, const Consts& k)
 {
-    if (!tma_requestable(D, method, k) || std::fabs(k.root_dpos) > 1e-14) return -1;
+    if (!tma_requestable(D, method, k) || (!fp32 && std::fabs(k.root_dpos) > 1e-14)) return -1;
     return k.limiter;
 }
 
@@ -69,7 +70,7 @@ bool tma_requestable(int D, int method, const Consts& k)
 cudaError_t launch_sweep(int D, int dir, int method, bool fp32, const SweepArgs& a, cudaStream_t s, bool march)
 {
     march = march && dir == 0 && D >= 2;
-    const void* fn = pick(D, dir, method, fp32, fast_limiter(D, method, a.k), march, a.rows);
+    const void* fn = pick(D, dir, method, fp32, fast_limiter(D, method, fp32, a.k), march, a.rows);
     if (!fn) return cudaErrorInvalidValue;
     if (a.total_items <= 0) return cudaSuccess;
     const int smem = march ? march_x_smem_bytes(D, fp32) : 0;
@@ -85,7 +86,7 @@ cudaError_t launch_sweep(int D, int dir, int method, bool fp32, const SweepArgs&
 long long sweep_resident_warps(int D, int dir, int method, bool fp32, const Consts& k, bool march)
 {
     march = march && dir == 0 && D >= 2;
-    const void* fn = pick(D, dir, method, fp32, fast_limiter(D, method, k), march, kRowsLevel);
+    const void* fn = pick(D, dir, method, fp32, fast_limiter(D, method, fp32, k), march, kRowsLevel);
     if (!fn) return 0;
     return (long long)device_sm_count() * blocks_per_sm(fn, march ? march_x_smem_bytes(D, fp32) : 0) *
            (kLaunchThreads / 32);

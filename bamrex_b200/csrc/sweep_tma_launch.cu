@@ -83,7 +83,7 @@ int blocks_per_sm(const void* fn, int smem, int threads)
 
 }  // namespace
 
-bool tma_supported(int D, int method, const Consts& k) { return D >= 2 && fast_limiter(D, method, k) >= 0; }
+bool tma_supported(int D, int method, bool fp32, const Consts& k) { return D >= 2 && fast_limiter(D, method, fp32, k) >= 0; }
 
 int tma_item_lines(bool wave, int dir) { return wave ? (dir == 0 ? WaveShape<double, 2, 0>::NL : WaveShape<double, 2, 1>::NL) : 32; }
 

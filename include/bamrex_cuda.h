@@ -215,9 +215,9 @@ typedef struct bamrex_level_desc {
  * its tiles arriving by tensor loads; cell stages and face fluxes pass
  * between threads through shared memory.  TMA and WAVE serve the fast
  * MUSCL-Hancock path in 2D and 3D (energy limiting, gamma with 1/z = 7);
- * other configurations refuse them with BAMREX_ERR_UNSUPPORTED (a gamma that
- * misses 1/z = 7 by more than its rounding, 1e-14, but by less than 1e-12 is
- * accepted and runs REGISTERS).  AUTO: x by REGISTERS, y and z per
+ * other configurations refuse them with BAMREX_ERR_UNSUPPORTED (in FP64 a
+ * gamma that misses 1/z = 7 by more than its rounding, 1e-14, but by less than
+ * 1e-12 is accepted and runs REGISTERS).  AUTO: x by REGISTERS, y and z per
  * direction the kind with the least estimated time on the level's boxes (a
  * slot-step count, warm-up and idle lanes included, times a time per
  * slot-step measured on the B200).  All evaluate the same scheme per cell
