@@ -93,8 +93,8 @@ __device__ __forceinline__ void phys_flux(const T (&U)[D + 2], const K<T>& k, T 
         const Prim<D, DIR> q(U, k);
         F[0] = U[1 + DIR];
 #pragma unroll
-        for (int d = 0; d < D; ++d) F[1 + d] = d == DIR ? fma(q.p, k.inv_eps, q.mnu) : U[1 + DIR] * q.u[d];
-        F[1 + D] = (U[1 + D] + q.p) * q.u[DIR];
+        for (int d = 0; d < D; ++d) F[1 + d] = d == DIR ? fma(q.p, k.inv_eps, q.mnu) : __dmul_rn(U[1 + DIR], q.u[d]);
+        F[1 + D] = __dmul_rn(U[1 + D] + q.p, q.u[DIR]);
     } else {
         T q[D + 2], ir;
         to_prim<T, D>(U, k, q, ir);
@@ -237,6 +237,13 @@ __device__ __forceinline__ void hllc_face(const T (&L)[D + 2], const T (&R)[D + 
     }
 }
 
+// FORCE and Lax-Friedrichs take the products of two neighbouring cells' fluxes
+// into sums; in FP64 each product and sum is spelled out, so that a face has
+// the same bits in whichever kernel, and whichever position of a lane, it is
+// formed (a level in boxes steps like one box).
+__device__ __forceinline__ double centred_sum(double a, double d, double s) { return fma(a, d, 0.5 * s); }
+__device__ __forceinline__ float centred_sum(float a, float d, float s) { return a * d + 0.5f * s; }
+
 // ---- face stage: FORCE (compute_force_flux_LR, Source/Fluxes/Force.cpp:22-108)
 template <typename T, int D, int DIR>
 __device__ __forceinline__ void force_face(const T (&L)[D + 2], const T (&R)[D + 2], const K<T>& k, T half_dx_dt,
@@ -248,8 +255,9 @@ __device__ __forceinline__ void force_face(const T (&L)[D + 2], const T (&R)[D +
     phys_flux<T, D, DIR>(R, k, fR);
 #pragma unroll
     for (int n = 0; n < NC; ++n) {
-        F[n] = T(0.5) * (half_dx_dt * (L[n] - R[n]) + T(0.5) * (fL[n] + fR[n]));
-        H[n] = T(0.5) * (L[n] + R[n]) + dt_2dx * (fL[n] - fR[n]);
+        F[n] = T(0.5) * centred_sum(half_dx_dt, L[n] - R[n], fL[n] + fR[n]);
+        if constexpr (sizeof(T) == 8) H[n] = centred_sum(dt_2dx, fL[n] - fR[n], L[n] + R[n]);
+        else H[n] = T(0.5) * (L[n] + R[n]) + dt_2dx * (fL[n] - fR[n]);
     }
     phys_flux<T, D, DIR>(H, k, fH);
 #pragma unroll
@@ -266,7 +274,7 @@ __device__ __forceinline__ void lf_face(const T (&L)[D + 2], const T (&R)[D + 2]
     phys_flux<T, D, DIR>(L, k, fL);
     phys_flux<T, D, DIR>(R, k, fR);
 #pragma unroll
-    for (int n = 0; n < NC; ++n) F[n] = half_dx_dt * (L[n] - R[n]) + T(0.5) * (fL[n] + fR[n]);
+    for (int n = 0; n < NC; ++n) F[n] = centred_sum(half_dx_dt, L[n] - R[n], fL[n] + fR[n]);
 }
 
 // |u| + c of a conserved state (max_wave_speed body, Euler.cpp:53-68).

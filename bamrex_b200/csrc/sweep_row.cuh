@@ -5,7 +5,7 @@
 // box given by value.
 //
 // Work decomposition.  A row's positions lo-2 .. hi+2 are cut into groups of
-// kP (4; 2 on the general path) and the groups of a box's rows are numbered
+// kP (row_group: 4 or 2) and the groups of a box's rows are numbered
 // one row after the other.  A chunk is 32 consecutive groups, one per lane;
 // lanes 1 .. 30 store their cells, lanes 0 and 31 are the halo of the chunk
 // (the neighbouring chunks own them).  A row carries its own halo positions,
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(kSweepThreads, row_min_blocks<T>()) sweep_row_
     using S = Scheme<T, D, 0, METHOD, LIM>;
     constexpr int NC = D + 2;
     constexpr int H = S::kHalo;
-    constexpr int kP = row_group(LIM);
+    constexpr int kP = row_group(METHOD, sizeof(T) == 4, LIM);
     constexpr int kPairs = kP / 2;
     static_assert(VEC || !LEVEL, "a level's rows are aligned to pairs");
     __shared__ Pair<T> stage[kSweepThreads / 32][2][NC][kPairs][32];
@@ -253,7 +253,12 @@ __global__ void __launch_bounds__(kSweepThreads, row_min_blocks<T>()) sweep_row_
                 S::cell(U[i], U[i + 1], U[i + 2], k, f.hdtdx, UL[i], UR[i]);
                 if (i) S::face(UR[i - 1], UL[i], k, f.half_dx_dt, f.dt_2dx, F[i]);
             }
-            shfl_up1(UR[kP - 1], URm);
+            if constexpr (S::kReconstruct) {
+                shfl_up1(UR[kP - 1], URm);
+            } else {  // the state itself, exchanged above
+#pragma unroll
+                for (int n = 0; n < NC; ++n) URm[n] = U[0][n];
+            }
             S::face(URm, UL[0], k, f.half_dx_dt, f.dt_2dx, F[0]);
             shfl_down1(F[0], F[kP]);
             T Un[kP][NC];
