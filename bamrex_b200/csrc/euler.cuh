@@ -238,11 +238,60 @@ __device__ __forceinline__ void hllc_face(const T (&L)[D + 2], const T (&R)[D + 
 }
 
 // FORCE and Lax-Friedrichs take the products of two neighbouring cells' fluxes
-// into sums; in FP64 each product and sum is spelled out, so that a face has
-// the same bits in whichever kernel, and whichever position of a lane, it is
-// formed (a level in boxes steps like one box).
+// into sums.  Every product and sum is spelled out, so that a face has the same
+// bits in whichever kernel, and whichever position of a lane, it is formed (a
+// level in boxes steps like one box); left to the compiler, the product that a
+// sum is contracted with depends on how often each is used around it.
+//
+// a d + s / 2
 __device__ __forceinline__ double centred_sum(double a, double d, double s) { return fma(a, d, 0.5 * s); }
-__device__ __forceinline__ float centred_sum(float a, float d, float s) { return a * d + 0.5f * s; }
+__device__ __forceinline__ float centred_sum(float a, float d, float s) { return fmaf(a, d, 0.5f * s); }
+
+// The sum and the difference of two states' fluxes.  FP32: each flux but the
+// mass and the normal momentum is a product, and the right one (LEFT: the
+// left one) enters unrounded, which are the bits FORCE and Lax-Friedrichs
+// have always had.
+template <int D, int DIR, bool LEFT>
+__device__ __forceinline__ void flux_pair(const double (&L)[D + 2], const double (&R)[D + 2], const K<double>& k,
+                                          double (&sum)[D + 2], double (&dif)[D + 2])
+{
+    double fL[D + 2], fR[D + 2];
+    phys_flux<double, D, DIR>(L, k, fL);
+    phys_flux<double, D, DIR>(R, k, fR);
+#pragma unroll
+    for (int n = 0; n < D + 2; ++n) {
+        sum[n] = fL[n] + fR[n];
+        dif[n] = fL[n] - fR[n];
+    }
+}
+template <int D, int DIR, bool LEFT>
+__device__ __forceinline__ void flux_pair(const float (&L)[D + 2], const float (&R)[D + 2], const K<float>& k,
+                                          float (&sum)[D + 2], float (&dif)[D + 2])
+{
+    constexpr int E = D + 1;
+    float qL[D + 2], qR[D + 2], ir;
+    to_prim<float, D>(L, k, qL, ir);
+    to_prim<float, D>(R, k, qR, ir);
+    sum[0] = L[1 + DIR] + R[1 + DIR];
+    dif[0] = L[1 + DIR] - R[1 + DIR];
+#pragma unroll
+    for (int n = 1; n < D + 2; ++n) {
+        // the flux as x y
+        const float xL = n == E ? L[E] + qL[E] : L[1 + DIR], yL = n == E ? qL[1 + DIR] : qL[n];
+        const float xR = n == E ? R[E] + qR[E] : R[1 + DIR], yR = n == E ? qR[1 + DIR] : qR[n];
+        if (n == 1 + DIR) {
+            const float a = fmaf(xL, yL, __fmul_rn(qL[E], k.inv_eps)), b = fmaf(xR, yR, __fmul_rn(qR[E], k.inv_eps));
+            sum[n] = a + b;
+            dif[n] = a - b;
+        } else if (LEFT) {
+            sum[n] = fmaf(xL, yL, __fmul_rn(xR, yR));
+            dif[n] = fmaf(xL, yL, -__fmul_rn(xR, yR));
+        } else {
+            sum[n] = fmaf(xR, yR, __fmul_rn(xL, yL));
+            dif[n] = fmaf(-xR, yR, __fmul_rn(xL, yL));
+        }
+    }
+}
 
 // ---- face stage: FORCE (compute_force_flux_LR, Source/Fluxes/Force.cpp:22-108)
 template <typename T, int D, int DIR>
@@ -250,14 +299,13 @@ __device__ __forceinline__ void force_face(const T (&L)[D + 2], const T (&R)[D +
                                            T dt_2dx, T (&F)[D + 2])
 {
     constexpr int NC = D + 2;
-    T fL[NC], fR[NC], H[NC], fH[NC];
-    phys_flux<T, D, DIR>(L, k, fL);
-    phys_flux<T, D, DIR>(R, k, fR);
+    T sum[NC], dif[NC], H[NC], fH[NC];
+    flux_pair<D, DIR, false>(L, R, k, sum, dif);
 #pragma unroll
     for (int n = 0; n < NC; ++n) {
-        F[n] = T(0.5) * centred_sum(half_dx_dt, L[n] - R[n], fL[n] + fR[n]);
-        if constexpr (sizeof(T) == 8) H[n] = centred_sum(dt_2dx, fL[n] - fR[n], L[n] + R[n]);
-        else H[n] = T(0.5) * (L[n] + R[n]) + dt_2dx * (fL[n] - fR[n]);
+        F[n] = T(0.5) * centred_sum(half_dx_dt, L[n] - R[n], sum[n]);
+        if constexpr (sizeof(T) == 8) H[n] = centred_sum(dt_2dx, dif[n], L[n] + R[n]);
+        else H[n] = fmaf(0.5f, L[n] + R[n], __fmul_rn(dt_2dx, dif[n]));
     }
     phys_flux<T, D, DIR>(H, k, fH);
 #pragma unroll
@@ -270,11 +318,10 @@ __device__ __forceinline__ void lf_face(const T (&L)[D + 2], const T (&R)[D + 2]
                                         T (&F)[D + 2])
 {
     constexpr int NC = D + 2;
-    T fL[NC], fR[NC];
-    phys_flux<T, D, DIR>(L, k, fL);
-    phys_flux<T, D, DIR>(R, k, fR);
+    T sum[NC], dif[NC];
+    flux_pair<D, DIR, true>(L, R, k, sum, dif);
 #pragma unroll
-    for (int n = 0; n < NC; ++n) F[n] = centred_sum(half_dx_dt, L[n] - R[n], fL[n] + fR[n]);
+    for (int n = 0; n < NC; ++n) F[n] = centred_sum(half_dx_dt, L[n] - R[n], sum[n]);
 }
 
 // |u| + c of a conserved state (max_wave_speed body, Euler.cpp:53-68).

@@ -35,9 +35,10 @@ def test_flux_and_update_by_width(oracle, D, shift, method):
             assert np.max(np.abs(new[n] - want[n])) <= RTOL * np.max(np.abs(want[n])), (w, n)
 
 
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "fp32_storage"])
 @pytest.mark.parametrize("method", [4, 5, 6], ids=["slic", "force", "lax_friedrichs"])
 @pytest.mark.parametrize("cuts", [[0, 64, 97, 128, 131, 200], [0, 2, 5, 66, 130], [0, 1, 4, 30, 60, 90, 120]])
-def test_boxes_step_like_one_box(cuts, method):
+def test_boxes_step_like_one_box(cuts, method, precision):
     """Boxes of even and odd widths step bit for bit like one box."""
     import bamrex_b200 as bx
     from bamrex_b200 import problems
@@ -47,7 +48,7 @@ def test_boxes_step_like_one_box(cuts, method):
     outs = []
     for boxes in ([((0, 0, 0), (nx - 1, ny - 1, 0))], parts):
         lev = bx.Level(2, (0, 0, 0), (nx - 1, ny - 1, 0), [0.0, 0.0], [1.0, 1.0], boxes, bx.Parm(2), method=method,
-                       cfl=0.6, bc_lo=(1,) * 3, bc_hi=(1,) * 3, x_mode=bx.XSWEEP_ROWS)
+                       cfl=0.6, bc_lo=(1,) * 3, bc_hi=(1,) * 3, x_mode=bx.XSWEEP_ROWS, precision=precision)
         lev.set_state(u0)
         lev.run(3, use_graph=False)
         outs.append(lev.get_state())
