@@ -531,7 +531,7 @@ static int per_box_sweep(int method, int dir, int D, const bamrex_box* bx, const
     const std::vector<bamrex_box> one(1, *bx);
     a.seglen = dir == 0 ? bx->hi[0] - bx->lo[0] + 1 : choose_seglen(dir, one, sweep_resident_warps(D, dir, method, false, k));
     long long items;
-    box_items(dir, B.lo, B.hi, a.seglen, items, B.nseg, B.ngroup, false, &B.seglen, row_positions(method, false, fast_limiter(D, method, false, k)));
+    box_items(dir, B.lo, B.hi, a.seglen, items, B.nseg, B.ngroup, false, &B.seglen, row_positions(method, fast_limiter(D, method, false, k)));
     // pairs of the row lie at an even distance from lo: aligned when cell lo
     // and the strides are
     auto paired = [&](const bamrex_array4& f) {
@@ -1101,7 +1101,7 @@ extern "C" int bamrex_level_create(bamrex_level** out, const bamrex_level_desc* 
     std::vector<SweepBox> sweep_host[3];
     // the register kernel of the x sweep when the caller leaves it open
     L->x_march = D >= 2 && (desc->x_mode == BAMREX_XSWEEP_MARCH || (desc->x_mode == BAMREX_XSWEEP_AUTO && narrow_rows(L->boxes)));
-    const int row_p = row_positions(L->method, L->fp32, fast_limiter(D, L->method, L->fp32, L->k));
+    const int row_p = row_positions(L->method, fast_limiter(D, L->method, L->fp32, L->k));
     for (int d = 0; d < D; ++d) {
         if (L->sweep_kind[d] >= 0) continue;
         if (!tma_supported(D, L->method, L->fp32, L->k)) {
@@ -1693,7 +1693,7 @@ int host_step_enqueue(bamrex_level* L, const double* host_in, double* host_out, 
         const bool march = dir == 0 && L->x_march;
         long long items;
         box_items(dir, sb.lo, sb.hi, L->seglen[dir], items, sb.nseg, sb.ngroup, march, &sb.seglen,
-                  row_positions(L->method, L->fp32, fast_limiter(D, L->method, L->fp32, L->k)));
+                  row_positions(L->method, fast_limiter(D, L->method, L->fp32, L->k)));
         sb.item_begin = 0;
         sa.total_items = items;
         sa.seglen = L->seglen[dir];

@@ -11,14 +11,13 @@ constexpr int kMaxComp = 8;
 
 // The x sweep by row groups (sweep_row.cuh): positions per lane and the groups
 // of a 32-lane chunk that store their cells.  Four positions on the fast path
-// and for FORCE and Lax-Friedrichs in FP64, whose arithmetic is little beside
-// the exchange of a group's edges (Lax-Friedrichs 2048^2 104 us with two, 72
-// with four; 256^3 in one box 505 and 342, in 32^3 boxes 667 and 432); two where
-// the general path's Riemann solves or reconstruction need the registers.  (FP32
-// storage keeps two there: four contract other multiply-adds.)
-__host__ __device__ constexpr int row_group(int method, bool fp32, int fast_lim)
+// and for FORCE and Lax-Friedrichs, whose arithmetic is little beside the
+// exchange of a group's edges (Lax-Friedrichs FP64 2048^2 104 us with two, 73
+// with four; 256^3 in one box 505 and 354, in 32^3 boxes 667 and 440); two where
+// the general path's Riemann solves or reconstruction need the registers.
+__host__ __device__ constexpr int row_group(int method, int fast_lim)
 {
-    return fast_lim >= 0 || (!fp32 && (method == BAMREX_FORCE || method == BAMREX_LAX_FRIEDRICHS)) ? 4 : 2;
+    return fast_lim >= 0 || method == BAMREX_FORCE || method == BAMREX_LAX_FRIEDRICHS ? 4 : 2;
 }
 constexpr int kRowOwned = 30;
 // Whose fabs that sweep works on: a level's, or one box of a caller's whose

@@ -61,6 +61,8 @@ template <int D, int DIR>
 struct Prim;
 
 // primv_from_consv (Source/System/Euler/Euler.H:167-198); inv_rho = 1/rho.
+// FP32 spells out its multiply-adds (here and in phys_flux), as the compiler
+// contracts them where nothing around competes for the products.
 template <typename T, int D>
 __device__ __forceinline__ void to_prim(const T (&U)[D + 2], const K<T>& k, T (&q)[D + 2], T& inv_rho)
 {
@@ -68,9 +70,15 @@ __device__ __forceinline__ void to_prim(const T (&U)[D + 2], const K<T>& k, T (&
     q[0] = U[0];
 #pragma unroll
     for (int d = 0; d < D; ++d) q[1 + d] = U[1 + d] * inv_rho;
-    T usq = q[1] * q[1];
+    T usq;
+    if constexpr (sizeof(T) == 4 && D > 1) {
+        usq = fmaf(q[1], q[1], __fmul_rn(q[2], q[2]));
+        if constexpr (D > 2) usq = fmaf(q[3], q[3], usq);
+    } else {
+        usq = q[1] * q[1];
 #pragma unroll
-    for (int d = 1; d < D; ++d) usq = usq + q[1 + d] * q[1 + d];
+        for (int d = 1; d < D; ++d) usq = usq + q[1 + d] * q[1 + d];
+    }
     q[1 + D] = k.gm1 * (U[1 + D] - k.half_eps * U[0] * usq);
 }
 
@@ -82,7 +90,8 @@ __device__ __forceinline__ void phys_flux(const T (&U)[D + 2], const T (&q)[D + 
     F[0] = mn;
 #pragma unroll
     for (int d = 0; d < D; ++d) F[1 + d] = mn * q[1 + d];
-    F[1 + DIR] += q[1 + D] * k.inv_eps;
+    if constexpr (sizeof(T) == 4) F[1 + DIR] = fmaf(mn, q[1 + DIR], __fmul_rn(q[1 + D], k.inv_eps));
+    else F[1 + DIR] += q[1 + D] * k.inv_eps;
     F[1 + D] = (U[1 + D] + q[1 + D]) * q[1 + DIR];
 }
 

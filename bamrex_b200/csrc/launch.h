@@ -78,7 +78,7 @@ int device_sm_count();
 
 // The x sweep by row groups (sweep_row.cuh): positions per lane (a row of n
 // cells is ceil((n + 4) / positions) groups; a chunk owns kRowOwned of them).
-inline int row_positions(int method, bool fp32, int fast_lim) { return row_group(method, fp32, fast_lim); }
+inline int row_positions(int method, int fast_lim) { return row_group(method, fast_lim); }
 
 // march: run the x sweep (dir 0, D >= 2) as one thread per row instead of
 // by row groups; the box table's items must be laid out to match (box_items).

@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(kSweepThreads, row_min_blocks<T>()) sweep_row_
     using S = Scheme<T, D, 0, METHOD, LIM>;
     constexpr int NC = D + 2;
     constexpr int H = S::kHalo;
-    constexpr int kP = row_group(METHOD, sizeof(T) == 4, LIM);
+    constexpr int kP = row_group(METHOD, LIM);
     constexpr int kPairs = kP / 2;
     static_assert(VEC || !LEVEL, "a level's rows are aligned to pairs");
     __shared__ Pair<T> stage[kSweepThreads / 32][2][NC][kPairs][32];
