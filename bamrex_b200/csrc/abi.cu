@@ -233,13 +233,38 @@ int choose_seglen(int dir, const std::vector<bamrex_box>& boxes, long long resid
     return best;
 }
 
-// Whether a level's rows are so short (24 cells or fewer on average) that the
-// marching x kernel serves it: a row of the row groups carries four halo
-// positions, and its halo lanes read the neighbours' rows.  3D 256^3, x sweep
-// by row groups / marching: FP64 in 64^3 boxes 566 / 650 us, 32^3 571 / 673,
-// 16^3 615 / 644, 8^3 894 / 850; FP32 32^3 300 / 433, 16^3 435 / 516, 240^3 in
-// 12^3 701 / 527; general path (gamma 5/3) 1024^2 FP64 in 64^2 boxes 52 / 53.
-bool narrow_rows(const std::vector<bamrex_box>& boxes)
+// The mean row length (cells) up to which the marching x kernel serves a
+// level's x sweep rather than the row groups, whose rows carry four halo
+// positions each and whose lanes beside a row's end read the neighbours' rows.
+// The lines lie where the two kernels' times cross (us, row groups / march; 3D
+// levels of about 200^3 in boxes of that width, the fast path's of 240^3):
+//  * fast path: FP64 10: 855 / 763, 12: 508 / 603, 16: 455 / 540, 24: 423 / 554;
+//    FP32 12: 653 / 523, 14: 544 / 493, 16: 323 / 429, 24: 254 / 375;
+//  * FORCE, Lax-Friedrichs: FP64 14: 237 / 216, 16: 221 / 233, 24: 217 / 270; FP32
+//    12: 340 / 285, 14: 187 / 233, 24: 135 / 208;  SLIC: FP64 16: 331 / 317, 18:
+//    286 / 308, FP32 12: 406 / 302, 16: 257 / 268;
+//  * HLLC: FP64 24: 345 / 322, 32: 331 / 317, 40: 194 / 201; FP32 24: 266 / 255, 32:
+//    252 / 245, 40: 149 / 156;
+//  * MUSCL-Hancock, general path: FP64 24: 411 / 400, 32: 392 / 387, 48: 376 / 402;
+//    FP32 32: 352 / 311, 48: 337 / 325, 64: 330 / 334; FP32 limited on several
+//    ratios, where the divisions of four cells crowd the row groups' registers,
+//    64: 597 / 493, one box of 192^3 562 / 451.
+// In 2D the row groups are faster at every width (FP64 2048^2 in 8^2 boxes 147 /
+// 338, 20^2 79 / 128, 32^2 118 / 152; FP32 16^2 96 / 160); FP64 levels of up to 20
+// cells keep the march, which x_mode reports for narrow levels.
+int march_rows(int D, int method, bool fp32, const Consts& k)
+{
+    if (D == 2) return fp32 ? 0 : 20;
+    if (fast_limiter(D, method, fp32, k) >= 0) return fp32 ? 14 : 12;
+    switch (method) {
+    case BAMREX_FORCE:
+    case BAMREX_LAX_FRIEDRICHS: return fp32 ? 12 : 14;
+    case BAMREX_SLIC: return 16;
+    case BAMREX_HLLC: return 32;
+    default: return !fp32 ? 24 : k.uniform_var >= 0 ? 40 : 1 << 20;
+    }
+}
+bool narrow_rows(const std::vector<bamrex_box>& boxes, long long limit)
 {
     long long cells = 0, rows = 0;
     for (const auto& b : boxes) {
@@ -247,7 +272,7 @@ bool narrow_rows(const std::vector<bamrex_box>& boxes)
         rows += r;
         cells += r * (b.hi[0] - b.lo[0] + 1);
     }
-    return cells <= 24 * rows;
+    return cells <= limit * rows;
 }
 
 // ---- TMA-staged sweeps (sweep_tma.cuh, sweep_wave.cuh): lane groups and
@@ -1100,7 +1125,7 @@ extern "C" int bamrex_level_create(bamrex_level** out, const bamrex_level_desc* 
     };
     std::vector<SweepBox> sweep_host[3];
     // the register kernel of the x sweep when the caller leaves it open
-    L->x_march = D >= 2 && (desc->x_mode == BAMREX_XSWEEP_MARCH || (desc->x_mode == BAMREX_XSWEEP_AUTO && narrow_rows(L->boxes)));
+    L->x_march = D >= 2 && (desc->x_mode == BAMREX_XSWEEP_MARCH || (desc->x_mode == BAMREX_XSWEEP_AUTO && narrow_rows(L->boxes, march_rows(D, L->method, L->fp32, L->k))));
     const int row_p = row_positions(L->method, fast_limiter(D, L->method, L->fp32, L->k));
     for (int d = 0; d < D; ++d) {
         if (L->sweep_kind[d] >= 0) continue;

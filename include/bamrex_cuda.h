@@ -230,10 +230,11 @@ enum {
 };
 
 /* Register kernel of a level's x sweep.  ROWS: row groups, each lane of a
- * warp on four consecutive cells of a row (two outside the fast path),
- * consecutive rows filling the warp.  MARCH: each thread marches one row,
- * lanes on 32 adjacent rows.  AUTO takes MARCH for levels whose rows are
- * 24 cells or shorter on average.  Both evaluate the same scheme per cell
+ * warp on four consecutive cells of a row (two for SLIC, HLLC and the general
+ * MUSCL-Hancock path), consecutive rows filling the warp.  MARCH: each thread
+ * marches one row, lanes on 32 adjacent rows.  AUTO takes MARCH for levels of short rows on
+ * average, by dimension, method and storage type (3D fast path: up to 12 cells
+ * in FP64, 14 in FP32 storage).  Both evaluate the same scheme per cell
  * (results agree to rounding: multiply-add contraction may differ). */
 enum {
     BAMREX_XSWEEP_AUTO = 0,
