@@ -318,7 +318,8 @@ __global__ void box_sums_kernel(int NC, const FabDev* __restrict__ fabs, const P
 }
 
 // ---------------------------------------------------------------- dt
-// estTimeStep (Source/AmrLevelAdv.cpp:395-477 -> FluidSystem.cpp:194-206):
+// estTimeStep (Source/AmrLevelAdv.cpp:395-477 -> FluidSystem.cpp:194-206) by
+// next_step_scalars (common.cuh): mode 0 of a run's start, 1 of a step's end.
 __global__ void step_dt_kernel(StepScalars* s, int D, double dx0, double dx1, double dx2, double cfl, int mode)
 {
     if (s->done) return;

@@ -25,10 +25,10 @@
 //
 // Measured on the B200 (x sweep, before -> now; before: the wavefront, a row
 // kernel with a carried pipeline or the marching kernel, whichever was
-// fastest): 4096^2 FP64 377 -> 357 us, in 64^2 boxes 482 -> 383, 256^3 in
-// 64^3 boxes 651 -> 465, in 32^3 674 -> 492; FP32 storage 4096^2 206 -> 177,
-// in 64^2 boxes 403 -> 217, 256^3 in 64^3 boxes 574 -> 242.  Bound by the
-// FP64 pipe (186 instructions per cell, 406 in all, half of the issue slots)
+// fastest): 4096^2 FP64 377 -> 359 us, in 64^2 boxes 482 -> 388, 256^3 in
+// 64^3 boxes 651 -> 466, in 32^3 674 -> 491; FP32 storage 4096^2 206 -> 174,
+// in 64^2 boxes 403 -> 213, 256^3 in 64^3 boxes 574 -> 241.  Bound by the
+// FP64 pipe (185 instructions per cell, 388 in all, half of the issue slots)
 // and the waits of two warps per scheduler.
 //
 // LEVEL: a level's own fabs (in and out laid out
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(kSweepThreads, row_min_blocks<T>()) sweep_row_
             T F[kP + 1][NC];  // faces x0 .. x0 + kP
             // cell after cell, each face as soon as its states are there and
             // the exchanged one last: the order the compiler overlaps best
-            // (4096^2 FP64 357 us; all cells first 409, the exchange early 404)
+            // (4096^2 FP64 357 us when tried; all cells first 409, the exchange early 404)
 #pragma unroll
             for (int i = 0; i < kP; ++i) {
                 S::cell(U[i], U[i + 1], U[i + 2], k, f.hdtdx, UL[i], UR[i]);
