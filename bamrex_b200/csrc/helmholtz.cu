@@ -1008,9 +1008,6 @@ int grid_for(long long n)
 struct bamrex_helmholtz {
     int D = 2;
     HOp op;
-    bool staged_smoother = true;  // 2D fused sweeps with cp.async-staged tiles
-    bool tiled_cycle = true;      // 2D levels above those: half a cycle per launch, in tiles
-    bool small_cycle = true;      // levels of <= 1024 cells cycled by one block in shared memory
     int nu1 = 2, nu2 = 2, bottom = 16;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
@@ -1090,7 +1087,7 @@ int smooth(bamrex_helmholtz* H, int l, int sweeps)
         const int tiles = (L.n[0] / kGsTX) * (L.n[1] / kGsTY);
         const int g = std::max(1, std::min(tiles, device_sm_count() * 8));
         // tiles staged by cp.async where the operator has no gradient term
-        const bool staged = L.c == nullptr && H->staged_smoother;
+        const bool staged = L.c == nullptr;
         if (staged) {
             static bool attr_set[64] = { false };
             int dev = 0;
@@ -1134,7 +1131,7 @@ int vcycle_phases(bamrex_helmholtz* H, int l);
 bool tiled_level(const bamrex_helmholtz* H, int l)
 {
     const HLev& L = H->lev[l];
-    return H->D == 2 && H->tiled_cycle && H->nu1 == 2 && H->nu2 == 2 && L.c == nullptr && l + 1 < (int)H->lev.size() &&
+    return H->D == 2 && H->nu1 == 2 && H->nu2 == 2 && L.c == nullptr && l + 1 < (int)H->lev.size() &&
            L.n[0] % 2 == 0 && L.n[1] % 2 == 0 && L.ncell > kSmallCells;
 }
 
@@ -1196,7 +1193,7 @@ int vcycle(bamrex_helmholtz* H, int l, const double* rhs, double* out, const dou
 int vcycle_phases(bamrex_helmholtz* H, int l)
 {
     const int nl = (int)H->lev.size();
-    if (H->small_cycle && H->lev[l].ncell <= kSmallCells && nl - l <= kSmallLevels) {
+    if (H->lev[l].ncell <= kSmallCells && nl - l <= kSmallLevels) {
         // the rest of the cycle in one block, its levels in shared memory
         HLevs lv;
         lv.n = nl - l;
